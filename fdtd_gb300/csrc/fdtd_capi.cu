@@ -92,15 +92,15 @@ static void cta_range(const Tiling &t, const int32_t lo[3], const int32_t hi[3],
     }
 }
 
-// CSR lists: for every CTA, the indices (into the device item array) of the
-// items whose box intersects the CTA's cells (and its halo), in item order.
-static void build_csr(const Tiling &t, const std::vector<ItemK> &items, int first, int count,
+// CSR lists: for every CTA, the indices (into the device item array) of those
+// items of `which` whose box intersects the CTA's cells (and its halo), in order.
+static void build_csr(const Tiling &t, const std::vector<ItemK> &items, const std::vector<int> &which,
                       std::vector<int> &off, std::vector<int> &idx, bool halo = false) {
     const long ncta = (long)t.gz * t.gy * t.gx;
     off.assign(ncta + 1, 0);
     idx.clear();
     std::vector<int> cnt(ncta, 0);
-    for (int q = first; q < first + count; ++q) {
+    for (int q : which) {
         int r[6];
         cta_range(t, items[q].lo, items[q].hi, r, halo);
         for (int cx = r[4]; cx <= r[5]; ++cx)
@@ -110,7 +110,7 @@ static void build_csr(const Tiling &t, const std::vector<ItemK> &items, int firs
     for (long c = 0; c < ncta; ++c) off[c + 1] = off[c] + cnt[c];
     idx.assign(off[ncta], 0);
     std::vector<int> fill(off.begin(), off.end() - 1);
-    for (int q = first; q < first + count; ++q) {
+    for (int q : which) {
         int r[6];
         cta_range(t, items[q].lo, items[q].hi, r, halo);
         for (int cx = r[4]; cx <= r[5]; ++cx)
@@ -765,10 +765,62 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
         }
     }
 
+    // what the fused passes apply, in order: the objects, and per half step the
+    // sources, a soft source of several points as one group (kItemSoftGroup)
+    struct Group {
+        int item;
+        std::vector<long long> cells;  // empty: the box is full
+        std::vector<double> weights;
+        size_t at_cells, at_weights;
+    };
+    std::vector<Group> groups;
+    std::vector<int> use_obj, use_src[2];
+    for (int q = 0; q < srcE0; ++q) use_obj.push_back(q);
+    for (int side = 0; side < 2; ++side) {
+        const int first = side == 0 ? srcE0 : srcH0;
+        const int last = first + (side == 0 ? d->n_sources_E : d->n_sources_H);
+        int e;
+        for (int q = first; q < last; q = e) {
+            e = q + 1;
+            while (e < last && items[e].source == items[q].source) ++e;
+            bool one = e - q > 1;
+            for (int r = q; r < e; ++r)
+                one = one && items[r].kind == FDTD_ITEM_SOFT && items[r].comp == items[q].comp &&
+                      items[r].column == items[q].column;
+            if (!one) {
+                for (int r = q; r < e; ++r) use_src[side].push_back(r);
+                continue;
+            }
+            Group gr;
+            ItemK it = items[q];
+            it.kind = kItemSoftGroup;
+            it.aux = e - q;
+            for (int r = q; r < e; ++r) {
+                for (int a = 0; a < 3; ++a) {
+                    it.lo[a] = std::min(it.lo[a], items[r].lo[a]);
+                    it.hi[a] = std::max(it.hi[a], items[r].hi[a]);
+                }
+                gr.cells.push_back(((long long)items[r].lo[0] * d->ny + items[r].lo[1]) * d->nz + items[r].lo[2]);
+                gr.weights.push_back(items[r].weight);
+            }
+            it.bny = it.hi[1] - it.lo[1];
+            it.bnz = it.hi[2] - it.lo[2];
+            // n distinct cells (they are sorted) in a box of n cells fill it, in box order
+            bool full = (long long)(it.hi[0] - it.lo[0]) * it.bny * it.bnz == (long long)gr.cells.size();
+            for (size_t r = 1; r < gr.cells.size(); ++r) full = full && gr.cells[r] != gr.cells[r - 1];
+            if (full) gr.cells.clear();
+            gr.item = (int)items.size();
+            use_src[side].push_back(gr.item);
+            items.push_back(it);
+            groups.push_back(gr);
+        }
+    }
+    const int ndev_items = (int)items.size();
+
     std::vector<int> obj_off, obj_idx, se_off, se_idx, sh_off, sh_idx;
-    build_csr(t, items, 0, srcE0, obj_off, obj_idx);
-    build_csr(t, items, srcE0, d->n_sources_E, se_off, se_idx);
-    build_csr(t, items, srcH0, d->n_sources_H, sh_off, sh_idx);
+    build_csr(t, items, use_obj, obj_off, obj_idx);
+    build_csr(t, items, use_src[0], se_off, se_idx);
+    build_csr(t, items, use_src[1], sh_off, sh_idx);
 
     // interior/shell partition: the boxes around the interior (x faces whole,
     // y faces within the interior's x range, z faces within its x and y
@@ -803,7 +855,7 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
         shk.first[shk.nbox] = (unsigned)blocks;
         // the blocks an item's cells fall in, ascending (rows of a box are
         // consecutive runs of cells, boxes follow one another)
-        auto lists = [&](int first, int count, std::vector<int> &off, std::vector<int> &idx) {
+        auto lists = [&](const std::vector<int> &which, std::vector<int> &off, std::vector<int> &idx) {
             off.assign(blocks + 1, 0);
             for (int pass = 0; pass < 2; ++pass) {
                 std::vector<int> fill;
@@ -812,7 +864,7 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
                     idx.assign(off[blocks], 0);
                     fill.assign(off.begin(), off.end() - 1);
                 }
-                for (int q = first; q < first + count; ++q) {
+                for (int q : which) {
                     const ItemK &it = items[q];
                     long last = -1;
                     for (int b = 0; b < shk.nbox; ++b) {
@@ -841,9 +893,9 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
                 }
             }
         };
-        lists(0, srcE0, shl[0], shl[1]);
-        lists(srcE0, d->n_sources_E, shl[2], shl[3]);
-        lists(srcH0, d->n_sources_H, shl[4], shl[5]);
+        lists(use_obj, shl[0], shl[1]);
+        lists(use_src[0], shl[2], shl[3]);
+        lists(use_src[1], shl[4], shl[5]);
         p.n_shell = shk.nbox;
     }
     size_t shell_ints = 0;
@@ -927,8 +979,8 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
         }
         if (per_x && d->nx < 4) refuse(5);
         if (per_x)
-            for (const ItemK &it : items)
-                if (it.lo[0] == 0 || it.hi[0] == d->nx) refuse(6);
+            for (int q = 0; q < nitems; ++q)
+                if (items[q].lo[0] == 0 || items[q].hi[0] == d->nx) refuse(6);
         const bool ok = why == 0;
         p.onepass_ok = ok ? 1 : 0;
         bool alt = d->E_alt != nullptr && d->H_alt != nullptr && aligned16(d->E_alt) && aligned16(d->H_alt);
@@ -1066,9 +1118,9 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
                     p.oblock = dim3(32, TY + 1, 1);
                     p.onepass = 1;
                     p.onepass_hcopy = per_x ? 1 : 0;
-                    build_csr(to, items, 0, srcE0, oo_off, oo_idx, true);
-                    build_csr(to, items, srcE0, d->n_sources_E, ose_off, ose_idx, true);
-                    build_csr(to, items, srcH0, d->n_sources_H, osh_off, osh_idx, true);
+                    build_csr(to, items, use_obj, oo_off, oo_idx, true);
+                    build_csr(to, items, use_src[0], ose_off, ose_idx, true);
+                    build_csr(to, items, use_src[1], osh_off, osh_idx, true);
                 } else {
                     p.onepass_why = 9;
                 }
@@ -1095,15 +1147,20 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
 
     // one device allocation for the plan's tables
     auto align = [](size_t v) { return (v + 255) & ~(size_t)255; };
-    const size_t b_items = align(sizeof(ItemK) * std::max(1, nitems));
+    const size_t b_items = align(sizeof(ItemK) * std::max(1, ndev_items));
     const size_t b_lists = align(sizeof(int) * (obj_off.size() + obj_idx.size() + se_off.size() + se_idx.size() +
                                                 sh_off.size() + sh_idx.size() + oo_off.size() + oo_idx.size() +
                                                 ose_off.size() + ose_idx.size() + osh_off.size() + osh_idx.size() +
                                                 cta_order.size() + 13 + shell_ints));
     const size_t b_runs = align(sizeof(int2) * std::max<size_t>(1, runs.size()));
     const size_t b_status = 512;  // status word; at +256 the persistent loop's barrier and tile counters
-    std::vector<char> host(b_items + b_lists + b_runs + b_status, 0);
-    if (nitems) memcpy(host.data(), items.data(), sizeof(ItemK) * nitems);
+    size_t b_groups = 0;
+    for (Group &gr : groups) {
+        gr.at_cells = b_items + b_lists + b_runs + b_status + b_groups;
+        gr.at_weights = gr.at_cells + sizeof(long long) * gr.cells.size();
+        b_groups += sizeof(long long) * gr.cells.size() + sizeof(double) * gr.weights.size();
+    }
+    std::vector<char> host(b_items + b_lists + b_runs + b_status + b_groups, 0);
     int *lists = (int *)(host.data() + b_items);
     size_t pos = 0;
     size_t at_obj_off, at_obj_idx, at_se_off, at_se_idx, at_sh_off, at_sh_idx;
@@ -1132,6 +1189,14 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
     if (!runs.empty()) memcpy(host.data() + b_items + b_lists, runs.data(), sizeof(int2) * runs.size());
     ce = cudaMalloc(&p.dev_mem, host.size());
     if (ce != cudaSuccess) return cuda_fail(ce);
+    for (const Group &gr : groups) {
+        if (!gr.cells.empty())
+            memcpy(host.data() + gr.at_cells, gr.cells.data(), sizeof(long long) * gr.cells.size());
+        memcpy(host.data() + gr.at_weights, gr.weights.data(), sizeof(double) * gr.weights.size());
+        items[gr.item].coef[0] = gr.cells.empty() ? nullptr : (const char *)p.dev_mem + gr.at_cells;
+        items[gr.item].coef[1] = (const char *)p.dev_mem + gr.at_weights;
+    }
+    if (ndev_items) memcpy(host.data(), items.data(), sizeof(ItemK) * ndev_items);
     ce = cudaMemcpy(p.dev_mem, host.data(), host.size(), cudaMemcpyHostToDevice);
     if (ce != cudaSuccess) {
         cudaFree(p.dev_mem);

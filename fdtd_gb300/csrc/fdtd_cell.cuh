@@ -186,6 +186,34 @@ __device__ __forceinline__ void apply_objects_v(const GridK &g, int i, int j, in
     }
 }
 
+// The points [a, b) of a soft source on cell (i, j, k) of its bounding box (a
+// cell may be listed more than once): its place in a box that is full, else
+// found by bisection.
+struct SoftSpan {
+    int a, b;
+};
+__device__ __forceinline__ SoftSpan soft_span(const GridK &g, const ItemK &s, int i, int j, int k) {
+    const long long *cells = (const long long *)s.coef[0];
+    if (cells == nullptr) {
+        const int a = (int)box_index(s, i, j, k);
+        return SoftSpan{a, a + 1};
+    }
+    const long long cell = ((long long)i * g.ny + j) * g.nz + k;
+    int a = 0, n = s.aux;
+    while (n > 0) {
+        const int h = n >> 1;
+        if (cells[a + h] < cell) {
+            a += h + 1;
+            n -= h + 1;
+        } else {
+            n = h;
+        }
+    }
+    int b = a;
+    while (b < s.aux && cells[b] == cell) ++b;
+    return SoftSpan{a, b};
+}
+
 // Sources of one cell (fdtd/sources.py:93-109, 278-297, 476-486), in order.
 template <class P>
 __device__ __forceinline__ void apply_sources(const GridK &g, const int *idx, const double *__restrict__ wave, int i,
@@ -196,7 +224,18 @@ __device__ __forceinline__ void apply_sources(const GridK &g, const int *idx, co
     for (int it = sb0; it < sb1; ++it) {
         const ItemK &s = g.items[idx[it]];
         if (!in_box(s, i, j, k)) continue;
-        const T w = (T)s.weight, wv = (T)wave[s.column];
+        const T wv = (T)wave[s.column];
+        if (s.kind == kItemSoftGroup) {
+            const SoftSpan q = soft_span(g, s, i, j, k);
+            for (int a = q.a; a < q.b; ++a) {
+                const T w = (T)((const double *)s.coef[1])[a];
+                if (s.comp == 0) P::add_prod(fx, lx, w, wv);
+                else if (s.comp == 1) P::add_prod(fy, ly, w, wv);
+                else P::add_prod(fz, lz, w, wv);
+            }
+            continue;
+        }
+        const T w = (T)s.weight;
         if (s.kind == FDTD_ITEM_SOFT) {
             if (s.comp == 0) P::add_prod(fx, lx, w, wv);
             else if (s.comp == 1) P::add_prod(fy, ly, w, wv);

@@ -37,8 +37,16 @@ struct ItemK {
     int bny, bnz;
     double weight;
     const void *coef[3];
-    int aux;  // FDTD_ITEM_FEEDBACK: its point in the current-probe list
+    int aux;  // FDTD_ITEM_FEEDBACK: its point in the current-probe list; kItemSoftGroup: its points
 };
+
+// All points of one soft source as one item of the fused passes: lo/hi their
+// bounding box, coef[0] their linear cells in ascending order (null: every
+// cell of the box exactly once, in box order), coef[1] their weights (double),
+// aux their number.  A line source of n points as n items had every thread of
+// its tiles test n boxes per plane: 2D 1500x1100 float32, a line of 550 cells,
+// 489 us per step against 41.7.
+constexpr int kItemSoftGroup = 100;
 
 // Material modes of a staged pass: the inverse material read per cell as
 // three values (MAT_FULL), as a one-byte index into a small table of value
