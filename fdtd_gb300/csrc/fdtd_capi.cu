@@ -2,6 +2,7 @@
 // descriptor validation, launch tiling, per-CTA object/source lists and
 // dispatch to the per-precision launch sequences.
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <mutex>
 #include <vector>
@@ -39,6 +40,60 @@ static int tile_width(int zt) {
     if (zt <= 32) return next_pow2(zt);
     const int pad32 = (zt + 31) / 32 * 32 - zt, pad16 = (zt + 15) / 16 * 16 - zt;
     return pad16 < pad32 ? 16 : 32;
+}
+
+// The layers of a flat pass by axis and side (GridK::lay); false where they
+// need the general form: two on one side, layers of one axis that share cells,
+// layers of two axes interleaved in boundary order, one behind a periodic
+// boundary, or auxiliaries that are not aligned to a pair.
+static bool flat_layers(GridK &g, size_t pair) {
+    bool ok = g.nslab_fused == g.nslab;
+    memset(g.lay, 0, sizeof(g.lay));
+    int axes[3], n = 0;
+    for (int s = 0; s < g.nslab; ++s) {
+        const SlabK &S = g.slab[s];
+        ok = ok && g.lay[S.axis][S.high].th == 0 && ((uintptr_t)S.psiE | (uintptr_t)S.psiH) % pair == 0;
+        g.lay[S.axis][S.high] = S;
+        int at = 0;
+        while (at < n && axes[at] != S.axis) ++at;
+        if (at == n) axes[n++] = S.axis;
+        else ok = ok && at == n - 1;
+    }
+    for (int a = 0; a < 3; ++a) {
+        ok = ok && (g.lay[a][0].th == 0 || g.lay[a][1].th == 0 || g.lay[a][0].th <= g.lay[a][1].start);
+        int at = 0;
+        while (at < n && axes[at] != a) ++at;
+        if (at == n) axes[n++] = a;
+    }
+    bool sorted = true;  // the plain order wherever it is as good as the registered one
+    for (int r = 0; r < 3; ++r) sorted = sorted && axes[r] == r;
+    g.lay_order = sorted ? 0x210 : (axes[0] | axes[1] << 4 | axes[2] << 8);
+    return ok;
+}
+
+// Planes per block of the flat half steps, for `wave` resident blocks: the
+// split whose waves of blocks take the fewest planes in all, a block counted
+// two planes more for its set-up.  Up to four waves count whole (a part-filled
+// last wave takes as long as a full one); at most 12 planes, or 16 in a single
+// wave, since blocks in layers are slower and long marches leave the last of
+// them alone.  us per step, float32: 128^3 16 planes (0.84 waves) 43, 8 (1.7)
+// 46, 12 (1.2) 49; 192x192x96 12 (1.9) 110, 16 (1.4) 121, 24 (0.95) 111;
+// 256^3 4, 8, 12, 16 planes 310, 301, 301, 304; 384x384x192 16 planes 665,
+// 23 765; 2D 4000^2 8, 12, 16, 32, 64 planes 273, 275, 281, 297, 315.
+static int flat_planes(int nx, long chunks, long wave) {
+    double best = 0.0;
+    int planes = 1;
+    for (int xc = 1; xc <= nx; ++xc) {
+        const long blocks = chunks * ((nx + xc - 1) / xc);
+        const double waves = (double)blocks / (double)wave;
+        if (xc > (waves > 1.0 ? 12 : 16) || (waves > 4.0 && xc < 6 && nx > 6)) continue;
+        const double cost = (waves > 4.0 ? waves : std::ceil(waves)) * (xc + 2);
+        if (best == 0.0 || cost < best) {
+            best = cost;
+            planes = xc;
+        }
+    }
+    return planes;
 }
 
 // Planes per CTA of the register-streaming kernels: at most 32, and fewer
@@ -116,6 +171,40 @@ static void build_csr(const Tiling &t, const std::vector<ItemK> &items, const st
         for (int cx = r[4]; cx <= r[5]; ++cx)
             for (int cy = r[2]; cy <= r[3]; ++cy)
                 for (int cz = r[0]; cz <= r[1]; ++cz) idx[fill[cz + t.gz * (cy + (long)t.gy * cx)]++] = q;
+    }
+}
+
+// The same for the flat half steps: per chunk of kFlatBlock cells of the
+// box's plane, the items that hold a cell of it on some plane of the box.
+static void flat_csr(const Tiling &t, long chunks, const std::vector<ItemK> &items, const std::vector<int> &which,
+                     std::vector<int> &off, std::vector<int> &idx) {
+    off.assign(chunks + 1, 0);
+    idx.clear();
+    const long row = t.e[2] - t.o[2];  // cells of a row of the box
+    std::vector<int> fill;
+    for (int pass = 0; pass < 2; ++pass) {
+        if (pass == 1) {
+            for (long c = 0; c < chunks; ++c) off[c + 1] += off[c];
+            idx.assign(off[chunks], 0);
+            fill.assign(off.begin(), off.end() - 1);
+        }
+        for (int q : which) {
+            int l[3], u[3];
+            for (int a = 0; a < 3; ++a) {
+                l[a] = std::max(items[q].lo[a], t.o[a]) - t.o[a];
+                u[a] = std::min(items[q].hi[a], t.e[a]) - t.o[a];
+            }
+            if (l[0] >= u[0] || l[1] >= u[1] || l[2] >= u[2]) continue;
+            long next = 0;  // rows come in order: the first chunk not yet listed
+            for (int y = l[1]; y < u[1]; ++y) {
+                const long b = (y * row + u[2] - 1) / kFlatBlock;
+                for (long c = std::max(next, (y * row + l[2]) / kFlatBlock); c <= b; ++c) {
+                    if (pass == 0) off[c + 1]++;
+                    else idx[fill[c]++] = q;
+                }
+                next = std::max(next, b + 1);
+            }
+        }
     }
 }
 
@@ -347,12 +436,13 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
     // CTAs that hold them late, and their auxiliary rows enlarge every stage.
     // The automatic choice therefore keeps only leading y slabs, for float32
     // with compact materials.
-    // 2D grids (nz = 1) of 8M cells and more split too (8192^2 float32: 63.1
-    // vs 58.0 Gcell/s with 32-plane chunks)
+    // 2D grids (nz = 1) of 8M cells and more split too, but for the flat half
+    // steps of float32 (4000^2, us per step: flat 275, split 332)
     p.pml_split = g.nslab > 0 && p.n_shell == 0 &&
                   (pml_base >= 2 ||
                    (pml_base == 0 && ncell >= (8L << 20) &&
-                    ((vec && (long)d->nz * 3 * (long)esize >= 768) || d->nz == 1)));
+                    ((vec && (long)d->nz * 3 * (long)esize >= 768) ||
+                     (d->nz == 1 && d->precision != FDTD_FLOAT32))));
     int kfs = 0;  // leading slabs kept in the fused pass when split
     const bool auto_keep = pml_base == 0 && d->precision == FDTD_FLOAT32 && mat_want[0] != MAT_FULL &&
                            mat_want[1] != MAT_FULL;
@@ -548,28 +638,29 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
                 pass_stages[pass] = sp;
             }
             stage_layout(t.TY, t.TZ);  // g.psi_off of the shared layout again
-            g.mat_E = mat_want[0];
-            g.mat_H = mat_want[1];
-            g.mlut_E = d->eps_table;
-            g.mlut_H = d->mu_table;
-            g.nlut_E = g.mat_E == MAT_FULL ? 0 : d->n_eps_table;
-            g.nlut_H = g.mat_H == MAT_FULL ? 0 : d->n_mu_table;
             g.lut_rows = lut_rows;
             p.index_E = d->eps_index;
             p.index_H = d->mu_index;
-            g.mid_E = g.mat_E == MAT_IDS ? d->eps_index : nullptr;
-            g.mid_H = g.mat_H == MAT_IDS ? d->mu_index : nullptr;
         }
     }
+    g.mat_E = mat_want[0];
+    g.mat_H = mat_want[1];
+    g.mlut_E = d->eps_table;
+    g.mlut_H = d->mu_table;
+    g.nlut_E = g.mat_E == MAT_FULL ? 0 : d->n_eps_table;
+    g.nlut_H = g.mat_H == MAT_FULL ? 0 : d->n_mu_table;
+    g.mid_E = g.mat_E == MAT_IDS ? d->eps_index : nullptr;
+    g.mid_H = g.mat_H == MAT_IDS ? d->mu_index : nullptr;
+    const bool flat = !use_tma && d->precision == FDTD_FLOAT32 && p.n_shell == 0;
+    p.flat = flat;
     if (!use_tma) {
-        t.V = vec ? vmax : 1;
-        const int zthreads0 = (bnz + t.V - 1) / t.V;
-        t.TZ = tile_width(zthreads0);
-        t.TY = kThreads / t.TZ;
+        t.V = vec && !flat ? vmax : 1;
+        t.TZ = flat ? kFlatBlock : tile_width((bnz + t.V - 1) / t.V);
+        t.TY = flat ? 1 : kThreads / t.TZ;
         g.stages = 0;
         p.variant = 1;
     }
-    if (p.n_shell) {
+    if (p.n_shell && !flat) {
         // the interior's last z tile: when less than half of it would be
         // active, its cells go to the shell (config 5 float32: z 32..172
         // would take three 64-cell tiles, the last 12 cells active; float32c:
@@ -581,10 +672,18 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
             t.e[2] = ibox[5];
         }
     }
-    const int zthreads = (bnz + t.V - 1) / t.V;
-    t.gz = (zthreads + t.TZ - 1) / t.TZ;
-    t.gy = (bny + t.TY - 1) / t.TY;
-    if (t.gy > 65535) return FDTD_ERR_UNSUPPORTED;
+    // flat: the tiling is counted in chunks of the plane
+    const long flat_chunks = ((long)bny * bnz + kFlatBlock - 1) / kFlatBlock;
+    if (!flat) {
+        const int zthreads = (bnz + t.V - 1) / t.V;
+        t.gz = (zthreads + t.TZ - 1) / t.TZ;
+        t.gy = (bny + t.TY - 1) / t.TY;
+        if (t.gy > 65535) return FDTD_ERR_UNSUPPORTED;
+    } else {
+        t.gz = (int)flat_chunks;
+        t.gy = 1;
+        g.flat_chunks = (unsigned)flat_chunks;
+    }
     if (d->x_chunk > 0) {
         t.XC = d->x_chunk;
     } else {
@@ -602,11 +701,11 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
             chunks = std::max(1L, std::min(chunks, std::max(1L, (long)bnx / 12)));
             t.XC = (int)((bnx + chunks - 1) / chunks);
         } else {
-            t.XC = register_chunk(bnx, cols, wave);
+            t.XC = flat ? flat_planes(bnx, flat_chunks, 4L * n_sm) : register_chunk(bnx, cols, wave);
         }
     }
     t.gx = (bnx + t.XC - 1) / t.XC;
-    if (t.gx > 65535) return FDTD_ERR_UNSUPPORTED;
+    if (flat ? flat_chunks * t.gx >= (1L << 31) : t.gx > 65535) return FDTD_ERR_UNSUPPORTED;
     // adjoint kernels: register streaming, tiled like the register kernels
     {
         const int V = vec ? vmax : 1;
@@ -638,7 +737,7 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
     g.TZ = t.TZ;
     g.TY = t.TY;
     g.XC = t.XC;
-    p.grid = dim3(t.gz, t.gy, t.gx);
+    p.grid = flat ? dim3((unsigned)(flat_chunks * t.gx), 1, 1) : dim3(t.gz, t.gy, t.gx);
     p.block = dim3(t.TZ, t.TY, 1);
 
     // items: objects, E sources, H sources
@@ -818,9 +917,15 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
     const int ndev_items = (int)items.size();
 
     std::vector<int> obj_off, obj_idx, se_off, se_idx, sh_off, sh_idx;
-    build_csr(t, items, use_obj, obj_off, obj_idx);
-    build_csr(t, items, use_src[0], se_off, se_idx);
-    build_csr(t, items, use_src[1], sh_off, sh_idx);
+    if (!flat) {
+        build_csr(t, items, use_obj, obj_off, obj_idx);
+        build_csr(t, items, use_src[0], se_off, se_idx);
+        build_csr(t, items, use_src[1], sh_off, sh_idx);
+    } else {
+        flat_csr(t, flat_chunks, items, use_obj, obj_off, obj_idx);
+        flat_csr(t, flat_chunks, items, use_src[0], se_off, se_idx);
+        flat_csr(t, flat_chunks, items, use_src[1], sh_off, sh_idx);
+    }
 
     // interior/shell partition: the boxes around the interior (x faces whole,
     // y faces within the interior's x range, z faces within its x and y
@@ -907,7 +1012,7 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
     // cells of the PML slabs inside the fused pass) first, so that they run
     // in the first waves instead of finishing last; the rest in grid order.
     std::vector<int> cta_order;
-    {
+    if (!flat) {
         const long ncta = (long)t.gz * t.gy * t.gx;
         const int zc = t.V * t.TZ;
         std::vector<double> extra(ncta, 0.0);
@@ -1197,6 +1302,13 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
         items[gr.item].coef[1] = (const char *)p.dev_mem + gr.at_weights;
     }
     if (ndev_items) memcpy(host.data(), items.data(), sizeof(ItemK) * ndev_items);
+    for (int side = 0; side < 2; ++side) {
+        FlatSources &f = side == 0 ? g.src_E : g.src_H;
+        const std::vector<int> &use = use_src[side];
+        f.n = use.size() <= kFlatSources ? (int)use.size() : -1;
+        if (!(side == 0 ? g.fuse_src_E : g.fuse_src_H)) f.n = 0;  // in kernels of their own
+        for (int q = 0; q < f.n; ++q) f.item[q] = items[use[q]];
+    }
     ce = cudaMemcpy(p.dev_mem, host.data(), host.size(), cudaMemcpyHostToDevice);
     if (ce != cudaSuccess) {
         cudaFree(p.dev_mem);
@@ -1214,7 +1326,7 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
     g.srcH_idx = dl + at_sh_idx;
     const int *order = cta_order.empty() ? nullptr : dl + at_order;
     g.cta_order = p.variant == 2 ? order : nullptr;
-    p.persist_order = p.variant == 1 ? order : nullptr;
+    p.persist_order = p.variant == 1 && !flat ? order : nullptr;
     p.runs = (const int2 *)(base + b_items + b_lists);
     g.status = (int *)(base + b_items + b_lists + b_runs);
     p.persist_bar = (unsigned *)(base + b_items + b_lists + b_runs + 256);
@@ -1269,6 +1381,7 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
         p.kf.ey = ibox[4];
         p.kf.ez = ibox[5];
     }
+    p.flat_general = flat && !flat_layers(p.kf, 2 * esize);
     p.kfH = p.kf;
     if (p.variant == 2) {
         GridK *pass_k[2] = {&p.kf, &p.kfH};
@@ -1345,13 +1458,13 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
     {
         int coop = 0;
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-        p.persist_ok = coop && p.variant == 1 && p.n_shell == 0 && p.epi_E.empty() && p.epi_H.empty() && !p.has_feedback &&
+        p.persist_ok = coop && p.variant == 1 && !p.flat_general && p.n_shell == 0 && p.epi_E.empty() && p.epi_H.empty() && !p.has_feedback &&
                        p.n_current == 0 && (int)p.dft.size() <= kPersistMaxDft;
-        // automatic: float32 below 3M cells, float64 below 8M (measured
-        // against one launch per half step, register tiles, 500 steps: 64^3
-        // with a 10-cell PML 1.54x float32 / 1.25x float64; 128^3 with PML
-        // and objects 1.03-1.12x; 192x192x96 with PML and an anisotropic box
-        // 0.985x float32, 1.07x float64)
+        // automatic: float32 and float32c below 3M cells, float64 below 8M.
+        // Against one launch per half step, flat tiles, us per step: 64^3
+        // 25.9 -> 14.4, 2D 1500x1100 43 -> 31, 128^3 55.6 -> 53.3, 131x150x97
+        // 55.7 -> 54.3, but 192x192x96 112 -> 135; float64 register tiles
+        // 64^3 1.25x, 192x192x96 1.07x
         const long auto_cells = d->precision == FDTD_FLOAT64 ? (8L << 20) : 3000000L;
         p.persistent = p.persist_ok && (d->persistent == 2 || (d->persistent == 0 && ncell < auto_cells));
         p.persist_blocks = 0;

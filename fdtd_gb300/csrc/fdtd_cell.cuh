@@ -192,13 +192,13 @@ __device__ __forceinline__ void apply_objects_v(const GridK &g, int i, int j, in
 struct SoftSpan {
     int a, b;
 };
-__device__ __forceinline__ SoftSpan soft_span(const GridK &g, const ItemK &s, int i, int j, int k) {
+__device__ __forceinline__ SoftSpan soft_span(const ItemK &s, int ny, int nz, int i, int j, int k) {
     const long long *cells = (const long long *)s.coef[0];
     if (cells == nullptr) {
         const int a = (int)box_index(s, i, j, k);
         return SoftSpan{a, a + 1};
     }
-    const long long cell = ((long long)i * g.ny + j) * g.nz + k;
+    const long long cell = ((long long)i * ny + j) * nz + k;
     int a = 0, n = s.aux;
     while (n > 0) {
         const int h = n >> 1;
@@ -226,7 +226,7 @@ __device__ __forceinline__ void apply_sources(const GridK &g, const int *idx, co
         if (!in_box(s, i, j, k)) continue;
         const T wv = (T)wave[s.column];
         if (s.kind == kItemSoftGroup) {
-            const SoftSpan q = soft_span(g, s, i, j, k);
+            const SoftSpan q = soft_span(s, g.ny, g.nz, i, j, k);
             for (int a = q.a; a < q.b; ++a) {
                 const T w = (T)((const double *)s.coef[1])[a];
                 if (s.comp == 0) P::add_prod(fx, lx, w, wv);

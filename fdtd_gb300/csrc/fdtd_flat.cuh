@@ -1,0 +1,606 @@
+// Flat half steps: one thread per cell, marching along x.
+//
+// A plane of a field is one contiguous run of ny nz cells.  A block takes
+// kFlatBlock consecutive cells of the tile box's plane and steps them through
+// a chunk of planes, so every lane holds a cell whatever nz is (odd extents,
+// 2D grids), a layer normal to z is a run of lanes and not a few lanes of
+// every warp, and a thread's place in the plane, its layers, their
+// coefficients and its neighbours' offsets are worked out once per chunk.
+// E marches up and H down, so the x neighbour is the plane before and stays in
+// registers.  The arithmetic of each cell and its order are those of thread_E
+// / thread_H, and so are the bits.
+//
+// Bound by latency and instruction issue, not by bytes: at 128^3 with 12-cell
+// layers (everything in L2) a half step issues 145 warp instructions per 32
+// cells, 37 % of the issue slots.  Four blocks of 64 registers per SM: five
+// (48 registers) and three (80, two planes in flight in every loop) measured
+// slower, 56 and 59 against 43 us per step.  Against the register-streaming
+// tiles (four cells per thread, whose warps all hold a few cells of each z
+// layer and whose 124 registers leave 16 warps per SM), float32, us per step:
+// 128^3 87 -> 53, 131x150x97 72 -> 56, 64^3 16.0 -> 14.4, 192x192x96 176 ->
+// 115.  With double or compensated values, and on the slab-free interior of a
+// partition, those stay faster: 256^3 float64 1416 against 1675, float32c 500
+// against 565.
+#pragma once
+
+#include "fdtd_cell.cuh"
+
+namespace fdtd {
+
+// Blocks per SM the kernels are compiled for, and whether the short loop loads
+// two planes before it computes the first (only where that leaves these blocks
+// resident).
+template <class P>
+struct FlatTune {
+    static constexpr int blocks = sizeof(typename P::T) == 8 ? 3 : 4;
+    static constexpr bool pairs = sizeof(typename P::T) == 4 && !P::COMP;
+};
+
+// A pair of auxiliaries of a layer, or of values.
+template <class T>
+struct alignas(2 * sizeof(T)) FlatPair {
+    T p0, p1;
+};
+
+// A thread's layer normal to one axis (q null: none): where the pair of the
+// present plane is, the coefficients, and whether the differences drive it
+// (not on the layer's plane whose neighbour lies outside it).
+template <class T>
+struct FlatLayer {
+    FlatPair<T> *q;
+    T b, c;
+    bool inc;
+};
+
+// The pair of a layer on one plane, updated with its two differences and stored.
+template <class P>
+__device__ __forceinline__ void flat_psi(const FlatLayer<typename P::T> &L, FlatPair<typename P::T> &p,
+                                         typename P::T d0, typename P::T d1) {
+    using T = typename P::T;
+    if constexpr (sizeof(T) == 4) {
+        // (without the drive: p b + 0 c)
+        p.p0 = P::psi(p.p0, L.b, L.inc ? d0 : T(0), L.c);
+        p.p1 = P::psi(p.p1, L.b, L.inc ? d1 : T(0), L.c);
+        if (L.q) *L.q = p;
+    } else if (L.q) {
+        if (L.inc) {
+            p.p0 = P::psi(p.p0, L.b, d0, L.c);
+            p.p1 = P::psi(p.p1, L.b, d1, L.c);
+        } else {
+            p.p0 = P::mul(p.p0, L.b);
+            p.p1 = P::mul(p.p1, L.b);
+        }
+        *L.q = p;
+    }
+}
+
+// Column of a block's thread in the plane of the tile box.
+struct FlatPlace {
+    bool in;
+    int j, k;
+};
+__device__ __forceinline__ FlatPlace flat_place(const GridK &g, unsigned chunk) {
+    const int bnz = g.ez - g.oz;
+    const long total = (long)(g.ey - g.oy) * bnz;
+    const long t = (long)chunk * kFlatBlock + threadIdx.x;
+    FlatPlace p;
+    p.in = t < total;
+    if (total < (1L << 31)) {
+        const unsigned row = (unsigned)t / (unsigned)bnz;
+        p.j = g.oy + (int)row;
+        p.k = g.oz + (int)((unsigned)t - row * (unsigned)bnz);
+    } else {
+        p.j = g.oy + (int)(t / bnz);
+        p.k = g.oz + (int)(t % bnz);
+    }
+    return p;
+}
+
+// The n sources in idx on the thread's cell of planes [xa, xb), in order, after
+// the march has stored those planes (compensated pairs not yet normalised).
+template <class P>
+__device__ __forceinline__ void flat_sources(const GridK &g, const int *idx, int n, const double *__restrict__ wave,
+                                             int xa, int xb, int j, int k, long jk, typename P::T *F,
+                                             typename P::T *Flo) {
+    using T = typename P::T;
+    for (int i = xa; i < xb; ++i) {
+        T *f = F + 3 * ((long)i * g.ny * g.nz + jk), *fl = P::COMP ? Flo + (f - F) : nullptr;
+        T y[3] = {T(0), T(0), T(0)};
+        if constexpr (P::COMP) {
+            for (int c = 0; c < 3; ++c) y[c] = fl[c];
+        }
+        for (int it = 0; it < n; ++it) {
+            const ItemK &s = g.items[idx[it]];
+            if (!in_box(s, i, j, k)) continue;
+            const int c = s.comp;
+            T x = f[c], l = c == 0 ? y[0] : (c == 1 ? y[1] : y[2]);
+            const T wv = (T)wave[s.column];
+            if (s.kind == kItemSoftGroup) {
+                const SoftSpan q = soft_span(s, g.ny, g.nz, i, j, k);
+                for (int a = q.a; a < q.b; ++a) P::add_prod(x, l, (T)((const double *)s.coef[1])[a], wv);
+            } else if (s.kind == FDTD_ITEM_SOFT) {
+                P::add_prod(x, l, (T)s.weight, wv);
+            } else {
+                P::set(x, l, P::mul((T)s.weight, wv));
+            }
+            f[c] = x;
+            if (c == 0) y[0] = l;
+            else if (c == 1) y[1] = l;
+            else y[2] = l;
+        }
+        if constexpr (P::COMP) {
+            for (int c = 0; c < 3; ++c) {
+                T x = f[c];
+                P::finish(x, y[c]);
+                f[c] = x;
+                fl[c] = y[c];
+            }
+        }
+    }
+}
+
+// Where a thread stands in its march: its cell of the present plane in the
+// neighbour field, the field, its compensation and the material (values or
+// index), and the neighbour field on the plane before.
+template <class T>
+struct FlatMarch {
+    const T *pn;
+    T *pf, *plo;
+    const T *pm;
+    const unsigned char *pid;
+    T by, bz;
+};
+
+// A cell of one plane: the neighbour field there and at its y and z
+// neighbours, the field, courant times the material.
+template <class T>
+struct FlatCell {
+    T ax, ay, az, yx, yz, zx, zy, f0, f1, f2, l0, l1, l2, m0, m1, m2;
+    int id;
+};
+
+// The loads of the cell `step` values on from the present plane's.
+template <class P, int MAT>
+__device__ __forceinline__ void flat_load(FlatCell<typename P::T> &v, const FlatMarch<typename P::T> &s, long step,
+                                          long istep, long oy, long oz) {
+    const typename P::T *n = s.pn + step, *f = s.pf + step;
+    v.ax = n[0];
+    v.ay = n[1];
+    v.az = n[2];
+    v.yx = n[oy];
+    v.yz = n[oy + 2];
+    v.zx = n[oz];
+    v.zy = n[oz + 1];
+    v.f0 = f[0];
+    v.f1 = f[1];
+    v.f2 = f[2];
+    v.l0 = v.l1 = v.l2 = typename P::T(0);
+    if constexpr (P::COMP) {
+        v.l0 = s.plo[step];
+        v.l1 = s.plo[step + 1];
+        v.l2 = s.plo[step + 2];
+    }
+    if constexpr (MAT == MAT_FULL) {
+        v.m0 = s.pm[step];
+        v.m1 = s.pm[step + 1];
+        v.m2 = s.pm[step + 2];
+    } else if constexpr (MAT == MAT_IDS) {
+        v.id = (int)s.pid[istep];
+    }
+}
+
+template <class P, int MAT>
+__device__ __forceinline__ void flat_material(FlatCell<typename P::T> &v, const typename P::T *lut, int nlut,
+                                              typename P::T courant, const typename P::T (&m)[3]) {
+    using T = typename P::T;
+    if constexpr (MAT == MAT_UNIFORM) {
+        v.m0 = m[0];
+        v.m1 = m[1];
+        v.m2 = m[2];
+    } else {
+        if constexpr (MAT == MAT_IDS) {
+            const bool in = v.id < nlut;  // an index past the table reads zeros
+            v.m0 = in ? lut[3 * v.id] : T(0);
+            v.m1 = in ? lut[3 * v.id + 1] : T(0);
+            v.m2 = in ? lut[3 * v.id + 2] : T(0);
+        }
+        v.m0 = P::cm(courant, v.m0);
+        v.m1 = P::cm(courant, v.m1);
+        v.m2 = P::cm(courant, v.m2);
+    }
+}
+
+template <class P, bool IS_E>
+__device__ __forceinline__ void flat_bulk(FlatCell<typename P::T> &v, typename P::T u0, typename P::T u1,
+                                          typename P::T u2) {
+    if (IS_E) {
+        P::add_prod(v.f0, v.l0, v.m0, u0);
+        P::add_prod(v.f1, v.l1, v.m1, u1);
+        P::add_prod(v.f2, v.l2, v.m2, u2);
+    } else {
+        P::sub_prod(v.f0, v.l0, v.m0, u0);
+        P::sub_prod(v.f1, v.l1, v.m1, u1);
+        P::sub_prod(v.f2, v.l2, v.m2, u2);
+    }
+}
+
+// Bulk update of a cell with all its neighbours in the grid, but for those
+// along z in a 2D grid; (by, bz) is the neighbour field on the plane before.
+template <class P, bool IS_E>
+__device__ __forceinline__ void flat_plain(FlatCell<typename P::T> &v, typename P::T by, typename P::T bz,
+                                           bool flat2d) {
+    using T = typename P::T;
+    const T xy = IS_E ? v.ay - by : by - v.ay, xz = IS_E ? v.az - bz : bz - v.az;
+    const T yx = IS_E ? v.ax - v.yx : v.yx - v.ax, yz = IS_E ? v.az - v.yz : v.yz - v.az;
+    const T zx = flat2d ? T(0) : (IS_E ? v.ax - v.zx : v.zx - v.ax);
+    const T zy = flat2d ? T(0) : (IS_E ? v.ay - v.zy : v.zy - v.ay);
+    flat_bulk<P, IS_E>(v, yz - zy, zx - xz, xy - yx);
+}
+
+// The cell stored, normalised unless sources follow.
+template <class P>
+__device__ __forceinline__ void flat_store(FlatCell<typename P::T> &v, const FlatMarch<typename P::T> &s, bool last,
+                                           long step) {
+    if (last) {
+        P::finish(v.f0, v.l0);
+        P::finish(v.f1, v.l1);
+        P::finish(v.f2, v.l2);
+    }
+    s.pf[step] = v.f0;
+    s.pf[step + 1] = v.f1;
+    s.pf[step + 2] = v.f2;
+    if constexpr (P::COMP) {
+        s.plo[step] = v.l0;
+        s.plo[step + 1] = v.l1;
+        s.plo[step + 2] = v.l2;
+    }
+}
+
+// The march moved on by `step` values past cell v.
+template <class P, int MAT>
+__device__ __forceinline__ void flat_next(FlatMarch<typename P::T> &s, const FlatCell<typename P::T> &v, long step,
+                                          long istep) {
+    s.by = v.ay;
+    s.bz = v.az;
+    s.pn += step;
+    s.pf += step;
+    if constexpr (P::COMP) s.plo += step;
+    if constexpr (MAT == MAT_FULL) s.pm += step;
+    if constexpr (MAT == MAT_IDS) s.pid += istep;
+}
+
+// The low or high layer of an axis at coordinate x: its slab-local index, -1 outside.
+__device__ __forceinline__ int flat_side(const SlabK (&lay)[2], int x, bool &low) {
+    low = x < lay[0].th;
+    const int l = x - lay[1].start;
+    return low ? x : (l >= 0 && l < lay[1].th ? l : -1);
+}
+
+template <class T, bool IS_E>
+__device__ __forceinline__ FlatLayer<T> flat_layer_at(const SlabK (&lay)[2], int l, bool low, long pair) {
+    const SlabK &A = lay[0], &B = lay[1];
+    FlatLayer<T> L;
+    L.q = (FlatPair<T> *)(IS_E ? (low ? A.psiE : B.psiE) : (low ? A.psiH : B.psiH)) + pair;
+    L.b = ((const T *)(IS_E ? (low ? A.bE : B.bE) : (low ? A.bH : B.bH)))[l];
+    L.c = ((const T *)(IS_E ? (low ? A.cE : B.cE) : (low ? A.cH : B.cH)))[l];
+    L.inc = IS_E ? l >= 1 : l <= (low ? A.th : B.th) - 2;
+    return L;
+}
+
+// One source on a cell of its box.
+template <class P>
+__device__ __forceinline__ void flat_source(const ItemK &s, int ny, int nz, const double *__restrict__ wave, int i,
+                                            int j, int k, FlatCell<typename P::T> &v) {
+    using T = typename P::T;
+    T x = s.comp == 0 ? v.f0 : (s.comp == 1 ? v.f1 : v.f2), l = s.comp == 0 ? v.l0 : (s.comp == 1 ? v.l1 : v.l2);
+    const T wv = (T)wave[s.column];
+    if (s.kind == kItemSoftGroup) {
+        const SoftSpan q = soft_span(s, ny, nz, i, j, k);
+        for (int a = q.a; a < q.b; ++a) P::add_prod(x, l, (T)((const double *)s.coef[1])[a], wv);
+    } else if (s.kind == FDTD_ITEM_SOFT) {
+        P::add_prod(x, l, (T)s.weight, wv);
+    } else {
+        P::set(x, l, P::mul((T)s.weight, wv));
+    }
+    if (s.comp == 0) {
+        v.f0 = x;
+        v.l0 = l;
+    } else if (s.comp == 1) {
+        v.f1 = x;
+        v.l1 = l;
+    } else {
+        v.f2 = x;
+        v.l2 = l;
+    }
+}
+
+// Planes [xa, xb) of a chunk of the plane.  A warp whose cells have all their
+// neighbours in the grid and lie in no layer and no object runs the short
+// loop, two planes loaded before the first is computed; the others run the
+// full one.
+template <class P, bool IS_E, int MAT>
+__device__ __forceinline__ void flat_tile(const GridK &g, const double *__restrict__ wave, unsigned chunk, int xa,
+                                          int xb) {
+    using T = typename P::T;
+    constexpr int dir = IS_E ? 1 : -1;
+    const int nx = g.nx, ny = g.ny, nz = g.nz;
+    const FlatPlace pl = flat_place(g, chunk);
+    const int j = pl.j, k = pl.k;
+    const long jk = (long)j * nz + k, nyz = (long)ny * nz;
+    const bool yok = IS_E ? j > 0 : j < ny - 1, zok = IS_E ? k > 0 : k < nz - 1;
+    // to the y and z neighbours (the cell itself where there is none)
+    const long oy = yok ? -dir * 3 * nz : 0, oz = zok ? -dir * 3 : 0;
+    const int i0 = IS_E ? xa : xb - 1;
+
+    // an object or source whose y and z ranges hold this cell sets a bit, so
+    // that a plane tests only those
+    int ob0 = 0, ob1 = 0;
+    unsigned omask = 0, smask = 0;
+    if constexpr (IS_E) {
+        ob0 = g.obj_off[chunk];
+        ob1 = g.obj_off[chunk + 1];
+        for (int it = ob0; it < min(ob1, ob0 + 32); ++it) {
+            const ItemK &o = g.items[g.obj_idx[it]];
+            if (o.lo[0] < xb && o.hi[0] > xa && j >= o.lo[1] && j < o.hi[1] && k >= o.lo[2] && k < o.hi[2])
+                omask |= 1u << (it - ob0);
+        }
+        ob1 = max(ob1, ob0 + 32);  // (past 32 the rest is tested plane by plane)
+    }
+    const FlatSources &src = IS_E ? g.src_E : g.src_H;
+    int listed = 0;  // more sources than the parameters hold: the chunk's list, after the march
+    if (src.n >= 0) {
+#pragma unroll
+        for (int q = 0; q < kFlatSources; ++q)
+            if (q < src.n && src.item[q].lo[0] < xb && src.item[q].hi[0] > xa && j >= src.item[q].lo[1] &&
+                j < src.item[q].hi[1] && k >= src.item[q].lo[2] && k < src.item[q].hi[2])
+                smask |= 1u << q;
+    } else {
+        const int *off = IS_E ? g.srcE_off : g.srcH_off;
+        listed = off[chunk + 1] - off[chunk];
+    }
+    bool ylow, zlow;
+    const int ly = flat_side(g.lay[1], j, ylow), lz = flat_side(g.lay[2], k, zlow);
+    const bool special =
+        __any_sync(0xffffffffu, pl.in && (!yok || (!zok && nz > 1) || ly >= 0 || lz >= 0 || omask != 0 || smask != 0 ||
+                                          ob1 > ob0 + 32));
+    if (!pl.in) return;
+
+    const T courant = courant_of<T>(g);
+    const T *lut = (const T *)(IS_E ? g.mlut_E : g.mlut_H);
+    const int nlut = IS_E ? g.nlut_E : g.nlut_H;
+    const long first = (long)i0 * nyz + jk, step = dir * 3 * nyz, istep = dir * nyz;
+    FlatMarch<T> s;
+    s.pn = (const T *)(IS_E ? g.H : g.E) + 3 * first;
+    s.pf = (T *)(IS_E ? g.E : g.H) + 3 * first;
+    s.plo = P::COMP ? (T *)(IS_E ? g.Elo : g.Hlo) + 3 * first : nullptr;
+    s.pm = MAT == MAT_FULL ? (const T *)(IS_E ? g.ie : g.imu) + 3 * first : nullptr;
+    s.pid = MAT == MAT_IDS ? (IS_E ? g.mid_E : g.mid_H) + first : nullptr;
+    T m[3] = {T(0), T(0), T(0)};
+    if constexpr (MAT == MAT_UNIFORM) {
+#pragma unroll
+        for (int q = 0; q < 3; ++q) m[q] = P::cm(courant, lut[q]);
+    }
+    bool xok = IS_E ? i0 > 0 : i0 < nx - 1;  // only the march's first plane can lack an x neighbour
+    s.by = s.bz = T(0);
+    if (xok) {
+        s.by = s.pn[1 - step];
+        s.bz = s.pn[2 - step];
+    }
+
+    FlatLayer<T> X{nullptr, T(0), T(0), false}, Y{nullptr, T(0), T(0), false}, W{nullptr, T(0), T(0), false};
+    int ystep = 0, wstep = 0;  // to the next plane's pair
+    if (special) {
+        if (ly >= 0) {
+            const int th = ylow ? g.lay[1][0].th : g.lay[1][1].th;
+            Y = flat_layer_at<T, IS_E>(g.lay[1], ly, ylow, ((long)i0 * th + ly) * nz + k);
+            ystep = dir * th * nz;
+        }
+        if (lz >= 0) {
+            const int thp = zlow ? g.lay[2][0].thp : g.lay[2][1].thp;
+            W = flat_layer_at<T, IS_E>(g.lay[2], lz, zlow, ((long)i0 * ny + j) * thp + lz);
+            wstep = dir * ny * thp;
+        }
+    }
+
+    const int end = IS_E ? xb : xa - 1;  // the march stops before this plane
+    int i = i0;
+    while (i != end) {
+        // planes up to the next face of a layer normal to x
+        int stop = end;
+        X.q = nullptr;
+        const T *tb = nullptr, *tc = nullptr;  // this layer's coefficients
+        int edge = -1;                         // its plane that no difference drives
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const SlabK &S = g.lay[0][h];
+            const int lo = S.start, hi = S.start + S.th;
+            if (lo == hi) continue;
+            if (i >= lo && i < hi) {
+                stop = IS_E ? min(stop, hi) : max(stop, lo - 1);
+                tb = (const T *)(IS_E ? S.bE : S.bH) - lo;
+                tc = (const T *)(IS_E ? S.cE : S.cH) - lo;
+                edge = IS_E ? lo : hi - 1;
+                X.q = (FlatPair<T> *)(IS_E ? S.psiE : S.psiH) + (long)(i - lo) * nyz + jk;
+            } else if (IS_E ? lo > i : hi <= i) {
+                stop = IS_E ? min(stop, lo) : max(stop, hi - 1);
+            }
+        }
+        if (!special && tb == nullptr && xok) {
+            if constexpr (FlatTune<P>::pairs) {
+#pragma unroll 1
+                for (; (stop - i) * dir >= 2; i += 2 * dir) {
+                    FlatCell<T> v, w;
+                    flat_load<P, MAT>(v, s, 0, 0, oy, oz);
+                    flat_load<P, MAT>(w, s, step, istep, oy, oz);
+                    flat_material<P, MAT>(v, lut, nlut, courant, m);
+                    flat_plain<P, IS_E>(v, s.by, s.bz, nz == 1);
+                    flat_store<P>(v, s, listed == 0, 0);
+                    flat_material<P, MAT>(w, lut, nlut, courant, m);
+                    flat_plain<P, IS_E>(w, v.ay, v.az, nz == 1);
+                    flat_store<P>(w, s, listed == 0, step);
+                    flat_next<P, MAT>(s, w, 2 * step, 2 * istep);
+                }
+            }
+#pragma unroll 1
+            for (; i != stop; i += dir) {
+                FlatCell<T> v;
+                flat_load<P, MAT>(v, s, 0, 0, oy, oz);
+                flat_material<P, MAT>(v, lut, nlut, courant, m);
+                flat_plain<P, IS_E>(v, s.by, s.bz, nz == 1);
+                flat_store<P>(v, s, listed == 0, 0);
+                flat_next<P, MAT>(s, v, step, istep);
+            }
+            continue;
+        }
+        const bool hx = tb != nullptr, hy = Y.q != nullptr, hw = W.q != nullptr;
+#pragma unroll 1
+        for (; i != stop; i += dir) {
+            FlatCell<T> v;
+            flat_load<P, MAT>(v, s, 0, 0, oy, oz);
+            FlatPair<T> qx{T(0), T(0)}, qy{T(0), T(0)}, qw{T(0), T(0)};
+            if (hx) {
+                qx = *X.q;
+                X.b = tb[i];
+                X.c = tc[i];
+                X.inc = i != edge;
+            }
+            if (hy) qy = *Y.q;
+            if (hw) qw = *W.q;
+            flat_material<P, MAT>(v, lut, nlut, courant, m);
+            // one-sided differences, zero where the neighbour is outside the grid
+            const T xy = xok ? (IS_E ? v.ay - s.by : s.by - v.ay) : T(0);
+            const T xz = xok ? (IS_E ? v.az - s.bz : s.bz - v.az) : T(0);
+            const T yx = yok ? (IS_E ? v.ax - v.yx : v.yx - v.ax) : T(0);
+            const T yz = yok ? (IS_E ? v.az - v.yz : v.yz - v.az) : T(0);
+            const T zx = zok ? (IS_E ? v.ax - v.zx : v.zx - v.ax) : T(0);
+            const T zy = zok ? (IS_E ? v.ay - v.zy : v.zy - v.ay) : T(0);
+            const T u0 = yz - zy, u1 = zx - xz, u2 = xy - yx;
+            flat_bulk<P, IS_E>(v, u0, u1, u2);
+            if constexpr (IS_E) {
+                for (unsigned om = omask; om; om &= om - 1) {
+                    const ItemK &o = g.items[g.obj_idx[ob0 + __ffs(om) - 1]];
+                    if (i >= o.lo[0] && i < o.hi[0])
+                        apply_object_cell<P>(o, box_index(o, i, j, k), courant, u0, u1, u2, v.f0, v.f1, v.f2, v.l0,
+                                             v.l1, v.l2);
+                }
+                for (int it = ob0 + 32; it < ob1; ++it) {
+                    const ItemK &o = g.items[g.obj_idx[it]];
+                    if (in_box(o, i, j, k))
+                        apply_object_cell<P>(o, box_index(o, i, j, k), courant, u0, u1, u2, v.f0, v.f1, v.f2, v.l0,
+                                             v.l1, v.l2);
+                }
+            }
+            // auxiliaries, then their corrections in boundary order (of a layer
+            // normal to c, component c+1 takes -p0 and c+2 takes p1)
+            if (hx) flat_psi<P>(X, qx, xz, xy);
+            flat_psi<P>(Y, qy, yx, yz);
+            flat_psi<P>(W, qw, zy, zx);
+            if (g.lay_order == 0x210) {
+                if (hx) pml_correct<P, IS_E>(v.f1, v.l1, v.m1, -qx.p0);
+                if (hx) pml_correct<P, IS_E>(v.f2, v.l2, v.m2, qx.p1);
+                if (hy) pml_correct<P, IS_E>(v.f2, v.l2, v.m2, -qy.p0);
+                if (hy) pml_correct<P, IS_E>(v.f0, v.l0, v.m0, qy.p1);
+                if (hw) pml_correct<P, IS_E>(v.f0, v.l0, v.m0, -qw.p0);
+                if (hw) pml_correct<P, IS_E>(v.f1, v.l1, v.m1, qw.p1);
+            } else {
+#pragma unroll 1
+                for (int o = g.lay_order, r = 0; r < 3; ++r, o >>= 4) {
+                    if ((o & 15) == 0 && hx) {
+                        pml_correct<P, IS_E>(v.f1, v.l1, v.m1, -qx.p0);
+                        pml_correct<P, IS_E>(v.f2, v.l2, v.m2, qx.p1);
+                    } else if ((o & 15) == 1 && hy) {
+                        pml_correct<P, IS_E>(v.f2, v.l2, v.m2, -qy.p0);
+                        pml_correct<P, IS_E>(v.f0, v.l0, v.m0, qy.p1);
+                    } else if ((o & 15) == 2 && hw) {
+                        pml_correct<P, IS_E>(v.f0, v.l0, v.m0, -qw.p0);
+                        pml_correct<P, IS_E>(v.f1, v.l1, v.m1, qw.p1);
+                    }
+                }
+            }
+            for (unsigned sm = smask; sm; sm &= sm - 1) {
+                const ItemK &o = src.item[__ffs(sm) - 1];
+                if (i >= o.lo[0] && i < o.hi[0]) flat_source<P>(o, ny, nz, wave, i, j, k, v);
+            }
+            flat_store<P>(v, s, listed == 0, 0);
+            flat_next<P, MAT>(s, v, step, istep);
+            X.q += istep;
+            if (hy) Y.q += ystep;
+            if (hw) W.q += wstep;
+            xok = true;
+        }
+    }
+    if (listed > 0) {
+        const int *idx = (IS_E ? g.srcE_idx : g.srcH_idx) + (IS_E ? g.srcE_off : g.srcH_off)[chunk];
+        flat_sources<P>(g, idx, listed, wave, xa, xb, j, k, jk, (T *)(IS_E ? g.E : g.H),
+                        (T *)(IS_E ? g.Elo : g.Hlo));
+    }
+}
+
+// The same with the per-cell body of the staged passes, which takes layers of
+// one axis that share cells, in any order and corrected later (a layer behind
+// a periodic boundary), and auxiliaries of any alignment.
+template <class P, bool IS_E>
+__device__ __forceinline__ void flat_tile_general(const GridK &g, const double *__restrict__ wave, unsigned chunk,
+                                                  int xa, int xb) {
+    using T = typename P::T;
+    const FlatPlace pl = flat_place(g, chunk);
+    if (!pl.in) return;
+    const int j = pl.j, k = pl.k, ny = g.ny, nz = g.nz;
+    const T *N = (const T *)(IS_E ? g.H : g.E);
+    T *F = (T *)(IS_E ? g.E : g.H);
+    T *Flo = (T *)(IS_E ? g.Elo : g.Hlo);
+    const T *M = (const T *)(IS_E ? g.ie : g.imu);
+    const T c = courant_of<T>(g);
+    const unsigned mask_yz = slab_mask_yz(g, j, k, 1);
+    const PsiSrc<T> nostage{nullptr, 0, 0, nullptr};
+    int sb0 = 0, sb1 = 0;
+    if (IS_E ? g.fuse_src_E : g.fuse_src_H) {
+        const int *off = IS_E ? g.srcE_off : g.srcH_off;
+        sb0 = off[chunk];
+        sb1 = off[chunk + 1];
+    }
+    for (int i = xa; i < xb; ++i) {
+        const long v = 3 * (((long)i * ny + j) * nz + k), d = IS_E ? -1 : 1;
+        T a[3], x[3] = {T(0), T(0), T(0)}, y[3] = {T(0), T(0), T(0)}, f[3], fl[3] = {T(0), T(0), T(0)}, m[3];
+        T kx = T(0), ky = T(0);
+        const bool xok = IS_E ? i > 0 : i < g.nx - 1, yok = IS_E ? j > 0 : j < ny - 1,
+                   zok = IS_E ? k > 0 : k < nz - 1;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            a[q] = N[v + q];
+            if (xok) x[q] = N[v + d * 3L * ny * nz + q];
+            if (yok) y[q] = N[v + d * 3L * nz + q];
+            f[q] = F[v + q];
+            if constexpr (P::COMP) fl[q] = Flo[v + q];
+            m[q] = M[v + q];
+        }
+        if (zok) {
+            kx = N[v + 3 * d];
+            ky = N[v + 3 * d + 1];
+        }
+        const unsigned slabs = mask_yz | slab_mask_x(g, i);
+        if constexpr (IS_E)
+            thread_E<P, 1>(g, wave, i, j, k, c, a, x, y, kx, ky, m, f, fl, g.obj_off[chunk], g.obj_off[chunk + 1], sb0,
+                           sb1, nostage, slabs);
+        else
+            thread_H<P, 1>(g, wave, i, j, k, c, a, x, y, kx, ky, m, f, fl, sb0, sb1, nostage, slabs);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            F[v + q] = f[q];
+            if constexpr (P::COMP) Flo[v + q] = fl[q];
+        }
+    }
+}
+
+// Block b of a half step: chunk b mod n of the plane, x chunk b / n.  MAT: how
+// the material is read, or -1 for the general form.
+template <class P, bool IS_E, int MAT>
+__global__ void __launch_bounds__(kFlatBlock, FlatTune<P>::blocks)
+    k_flat(const __grid_constant__ GridK g, const double *__restrict__ wave) {
+    const unsigned n = g.flat_chunks, xc = blockIdx.x / n, chunk = blockIdx.x - xc * n;
+    const int xa = g.ox + (int)xc * g.XC, xb = min(g.ex, xa + g.XC);
+    if constexpr (MAT < 0) flat_tile_general<P, IS_E>(g, wave, chunk, xa, xb);
+    else flat_tile<P, IS_E, MAT>(g, wave, chunk, xa, xb);
+}
+
+}  // namespace fdtd

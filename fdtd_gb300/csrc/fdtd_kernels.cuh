@@ -1,15 +1,15 @@
 // Kernels of the GB300 FDTD time step.
 //
-// k_update_E / k_update_H are the fused half steps.  One pass per half step
-// does, per cell and in the reference's order (fdtd/grid.py:275-325):
+// The fused half steps (fdtd_flat.cuh, fdtd_tma.cuh) do, per cell and in the
+// reference's order (fdtd/grid.py:275-325):
 //   PML auxiliary update (fdtd/boundaries.py:433-487, slab-local index rules)
 //   Yee curl (fdtd/grid.py:29-76, out-of-grid differences dropped)
 //   bulk update E += c*eps^-1*curlH / H -= c*mu^-1*curlE
 //   objects in registration order (fdtd/objects.py:118-277)
 //   PML corrections in boundary order (fdtd/boundaries.py:409-431)
 //   sources in registration order (fdtd/sources.py:93-109,278-297,476-486)
-// A CTA covers TZ*V cells along z, TY rows along y and XC planes along x; a
-// thread streams along x holding the neighbour plane in registers.
+// Here: the shell of a partition, PML slabs on their own, what runs between
+// the half steps, detectors, stand-alone curls and statistics.
 #pragma once
 
 #include "fdtd_cell.cuh"
@@ -18,14 +18,19 @@ namespace fdtd {
 
 #define FULL_MASK 0xffffffffu
 
-// Register-streaming kernels: neighbour values come from global memory
+// Register-streaming kernels (float64, float32c, and the interior of a float32
+// partition; other float32 grids have the flat half steps): neighbour values
+// come from global memory
 // (L1/L2) and from the lane to the left/right; used for shapes the staged
 // kernels do not take (nz not a multiple of the vector width, unaligned data).
 // One tile of the E half (bx, by, bz: tile coordinates; cta: its index in the
 // per-CTA lists), for the one-tile-per-block kernel and the persistent one.
 // CG: the other half's field is written by other blocks of the same launch
 // (persistent loop), so it is loaded through L2 only, not the read-only path.
-template <class P, int V, bool CG = false>
+// MAT_UNIFORM: every cell holds the same material, which is not read per cell
+// (the permeability of most grids; 256^3 random permittivity with a 16-cell
+// shell, float32: 381 -> 361 us per step).
+template <class P, int V, bool CG = false, int MAT = MAT_FULL>
 __device__ __forceinline__ void tile_update_E(const GridK &g, const double *__restrict__ wave, int bx, int by, int bz,
                                               int cta) {
     using T = typename P::T;
@@ -49,6 +54,11 @@ __device__ __forceinline__ void tile_update_E(const GridK &g, const double *__re
         sb1 = g.srcE_off[cta + 1];
     }
 
+    T mu[3] = {T(0), T(0), T(0)};
+    if constexpr (MAT == MAT_UNIFORM) {
+#pragma unroll
+        for (int q = 0; q < 3; ++q) mu[q] = __ldg((const T *)g.mlut_E + q);
+    }
     const PsiSrc<T> nostage{nullptr, 0, 0, nullptr};
     const unsigned mask_yz = slab_mask_yz(g, j, k0, V);
     alignas(16) T hp[N];  // H at plane i-1
@@ -65,14 +75,14 @@ __device__ __forceinline__ void tile_update_E(const GridK &g, const double *__re
             hj[q] = T(0);
             e[q] = T(0);
             el[q] = T(0);
-            m[q] = T(0);
+            m[q] = MAT == MAT_UNIFORM ? mu[q % 3] : T(0);
         }
         if (act) {
             ld_field<CG>(hc, H + 3 * cell0);
             if (j > 0) ld_field<CG>(hj, H + 3 * (cell0 - nz));
             ld_vec(e, E + 3 * cell0);
             if constexpr (P::COMP) ld_vec(el, Elo + 3 * cell0);
-            ld_vec_ro(m, IE + 3 * cell0);
+            if constexpr (MAT == MAT_FULL) ld_vec_ro(m, IE + 3 * cell0);
         }
         // (Hx, Hy) at k0-1: from the lane to the left, or from memory at a row start
         T kx = __shfl_up_sync(FULL_MASK, hc[N - 3], 1);
@@ -92,13 +102,13 @@ __device__ __forceinline__ void tile_update_E(const GridK &g, const double *__re
     }
 }
 
-template <class P, int V>
+template <class P, int V, int MAT>
 __global__ void __launch_bounds__(kThreads) k_update_E(const GridK g, const double *__restrict__ wave) {
-    tile_update_E<P, V>(g, wave, blockIdx.x, blockIdx.y, blockIdx.z,
+    tile_update_E<P, V, false, MAT>(g, wave, blockIdx.x, blockIdx.y, blockIdx.z,
                         blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z));
 }
 
-template <class P, int V, bool CG = false>
+template <class P, int V, bool CG = false, int MAT = MAT_FULL>
 __device__ __forceinline__ void tile_update_H(const GridK &g, const double *__restrict__ wave, int bx, int by, int bz,
                                               int cta) {
     using T = typename P::T;
@@ -121,6 +131,11 @@ __device__ __forceinline__ void tile_update_H(const GridK &g, const double *__re
         sb1 = g.srcH_off[cta + 1];
     }
 
+    T mu[3] = {T(0), T(0), T(0)};
+    if constexpr (MAT == MAT_UNIFORM) {
+#pragma unroll
+        for (int q = 0; q < 3; ++q) mu[q] = __ldg((const T *)g.mlut_H + q);
+    }
     const PsiSrc<T> nostage{nullptr, 0, 0, nullptr};
     const unsigned mask_yz = slab_mask_yz(g, j, k0, V);
     alignas(16) T ec[N];  // E at plane i
@@ -137,14 +152,14 @@ __device__ __forceinline__ void tile_update_H(const GridK &g, const double *__re
             ej[q] = T(0);
             h[q] = T(0);
             hl[q] = T(0);
-            m[q] = T(0);
+            m[q] = MAT == MAT_UNIFORM ? mu[q % 3] : T(0);
         }
         if (act) {
             if (i + 1 < nx) ld_field<CG>(en, E + 3 * (cell0 + (size_t)ny * nz));
             if (j + 1 < ny) ld_field<CG>(ej, E + 3 * (cell0 + nz));
             ld_vec(h, H + 3 * cell0);
             if constexpr (P::COMP) ld_vec(hl, Hlo + 3 * cell0);
-            ld_vec_ro(m, MU + 3 * cell0);
+            if constexpr (MAT == MAT_FULL) ld_vec_ro(m, MU + 3 * cell0);
         }
         // (Ex, Ey) at k0+V: from the lane to the right, or from memory at a row end
         T kx = __shfl_down_sync(FULL_MASK, ec[0], 1);
@@ -165,9 +180,9 @@ __device__ __forceinline__ void tile_update_H(const GridK &g, const double *__re
     }
 }
 
-template <class P, int V>
+template <class P, int V, int MAT>
 __global__ void __launch_bounds__(kThreads) k_update_H(const GridK g, const double *__restrict__ wave) {
-    tile_update_H<P, V>(g, wave, blockIdx.x, blockIdx.y, blockIdx.z,
+    tile_update_H<P, V, false, MAT>(g, wave, blockIdx.x, blockIdx.y, blockIdx.z,
                         blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z));
 }
 

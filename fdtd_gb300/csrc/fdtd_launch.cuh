@@ -6,6 +6,7 @@
 #include <type_traits>
 
 #include "fdtd_adjoint.cuh"
+#include "fdtd_flat.cuh"
 #include "fdtd_kernels.cuh"
 #include "fdtd_persistent.cuh"
 #include "fdtd_plan.hpp"
@@ -70,6 +71,31 @@ static void launch_tma(Plan &p, bool is_E, const double *wave, cudaStream_t st) 
     }
 }
 
+// Register-streaming half steps: a uniform material is not read per cell, an
+// indexed one is read in full.
+template <class P, int V>
+static void launch_register(Plan &p, bool is_E, const double *wave, cudaStream_t st) {
+    if (is_E && p.kf.mat_E == MAT_UNIFORM) k_update_E<P, V, MAT_UNIFORM><<<p.grid, p.block, 0, st>>>(p.kf, wave);
+    else if (is_E) k_update_E<P, V, MAT_FULL><<<p.grid, p.block, 0, st>>>(p.kf, wave);
+    else if (p.kf.mat_H == MAT_UNIFORM) k_update_H<P, V, MAT_UNIFORM><<<p.grid, p.block, 0, st>>>(p.kf, wave);
+    else k_update_H<P, V, MAT_FULL><<<p.grid, p.block, 0, st>>>(p.kf, wave);
+}
+
+template <class P, int MAT>
+static void launch_flat_mat(Plan &p, bool is_E, const double *wave, cudaStream_t st) {
+    if (is_E) k_flat<P, true, MAT><<<p.grid, kFlatBlock, 0, st>>>(p.kf, wave);
+    else k_flat<P, false, MAT><<<p.grid, kFlatBlock, 0, st>>>(p.kf, wave);
+}
+
+template <class P>
+static void launch_flat(Plan &p, bool is_E, const double *wave, cudaStream_t st) {
+    const int mat = p.flat_general ? -1 : (is_E ? p.kf.mat_E : p.kf.mat_H);
+    if (mat < 0) launch_flat_mat<P, -1>(p, is_E, wave, st);
+    else if (mat == MAT_UNIFORM) launch_flat_mat<P, MAT_UNIFORM>(p, is_E, wave, st);
+    else if (mat == MAT_IDS) launch_flat_mat<P, MAT_IDS>(p, is_E, wave, st);
+    else launch_flat_mat<P, MAT_FULL>(p, is_E, wave, st);
+}
+
 // Staged-kernel tile shapes (threads along z x rows): 32x8, 32x4, 16x16.
 // The fused pass of a half step: one launch over the tile box and, for a
 // partitioned plan, one launch over the shell boxes, on the plan's second
@@ -78,7 +104,6 @@ static void launch_tma(Plan &p, bool is_E, const double *wave, cudaStream_t st) 
 // field).
 template <class P>
 static void launch_fused(Plan &p, bool is_E, const double *wave, cudaStream_t st) {
-    constexpr int VV = P::V;
     if (p.n_shell && p.shell_overlap) {
         cudaEventRecord(p.shell_fork, st);
         cudaStreamWaitEvent(p.shell_stream, p.shell_fork, 0);
@@ -87,12 +112,12 @@ static void launch_fused(Plan &p, bool is_E, const double *wave, cudaStream_t st
         if (p.kf.TY == 16) launch_tma<P, 16, 16>(p, is_E, wave, st);
         else if (p.kf.TY == 8) launch_tma<P, 32, 8>(p, is_E, wave, st);
         else launch_tma<P, 32, 4>(p, is_E, wave, st);
+    } else if (p.flat) {
+        if constexpr (std::is_same<P, PF32>::value) launch_flat<P>(p, is_E, wave, st);
     } else if (p.V == 1) {
-        if (is_E) k_update_E<P, 1><<<p.grid, p.block, 0, st>>>(p.kf, wave);
-        else k_update_H<P, 1><<<p.grid, p.block, 0, st>>>(p.kf, wave);
+        launch_register<P, 1>(p, is_E, wave, st);
     } else {
-        if (is_E) k_update_E<P, VV><<<p.grid, p.block, 0, st>>>(p.kf, wave);
-        else k_update_H<P, VV><<<p.grid, p.block, 0, st>>>(p.kf, wave);
+        launch_register<P, P::V>(p, is_E, wave, st);
     }
     if (p.n_shell) {
         const unsigned blocks = p.shellk.first[p.shellk.nbox];
@@ -281,6 +306,20 @@ static size_t stage_bytes_of(int tile_rows, int mat_E, int mat_H) {
     return a > b ? a : b;
 }
 
+// The persistent loop over flat tiles for a plan's two material modes (an
+// indexed H material is read in full).
+template <class P>
+static const void *persist_flat(int mat_E, int mat_H) {
+    if (mat_H == MAT_UNIFORM) {
+        if (mat_E == MAT_UNIFORM) return (const void *)k_run_persistent<P, 0, MAT_UNIFORM, MAT_UNIFORM>;
+        if (mat_E == MAT_IDS) return (const void *)k_run_persistent<P, 0, MAT_IDS, MAT_UNIFORM>;
+        return (const void *)k_run_persistent<P, 0, MAT_FULL, MAT_UNIFORM>;
+    }
+    if (mat_E == MAT_UNIFORM) return (const void *)k_run_persistent<P, 0, MAT_UNIFORM, MAT_FULL>;
+    if (mat_E == MAT_IDS) return (const void *)k_run_persistent<P, 0, MAT_IDS, MAT_FULL>;
+    return (const void *)k_run_persistent<P, 0, MAT_FULL, MAT_FULL>;
+}
+
 // All steps of a call in one cooperative launch (fdtd_persistent.cuh).
 template <class P>
 static int run_persistent(Plan &p, const fdtd_run_args *a, bool detect, cudaStream_t st) {
@@ -288,9 +327,6 @@ static int run_persistent(Plan &p, const fdtd_run_args *a, bool detect, cudaStre
     pa.n_steps = a->n_steps;
     pa.wave = a->wave;
     pa.n_columns = p.n_columns;
-    pa.gz = (int)p.grid.x;
-    pa.gy = (int)p.grid.y;
-    pa.gx = (int)p.grid.z;
     pa.n_probe = detect ? p.n_probe : 0;
     pa.probe_cells = p.probe_cells;
     if (pa.n_probe) {
@@ -305,8 +341,18 @@ static int run_persistent(Plan &p, const fdtd_run_args *a, bool detect, cudaStre
     pa.tickets = p.persist_tickets;
     pa.order = p.persist_order;
     pa.limit = 1u << 23;
-    const bool vec = p.V > 1;
-    const void *fn = vec ? (const void *)k_run_persistent<P, P::V> : (const void *)k_run_persistent<P, 1>;
+    const void *fn = nullptr;
+    dim3 block = p.block;
+    if constexpr (std::is_same<P, PF32>::value) {
+        fn = persist_flat<P>(p.kf.mat_E, p.kf.mat_H);
+        block = dim3(kFlatBlock);
+    } else if (p.kf.mat_H == MAT_UNIFORM) {
+        fn = p.V > 1 ? (const void *)k_run_persistent<P, P::V, MAT_FULL, MAT_UNIFORM>
+                     : (const void *)k_run_persistent<P, 1, MAT_FULL, MAT_UNIFORM>;
+    } else {
+        fn = p.V > 1 ? (const void *)k_run_persistent<P, P::V, MAT_FULL, MAT_FULL>
+                     : (const void *)k_run_persistent<P, 1, MAT_FULL, MAT_FULL>;
+    }
     if (p.persist_blocks == 0) {
         int per_sm = 0, dev = 0, n_sm = 0;
         cudaGetDevice(&dev);
@@ -318,14 +364,25 @@ static int run_persistent(Plan &p, const fdtd_run_args *a, bool detect, cudaStre
         }
         p.persist_blocks = per_sm * n_sm;
     }
-    const int tiles = (int)(p.grid.x * p.grid.y * p.grid.z);
-    const int blocks = std::min(tiles, p.persist_blocks);
+    pa.gz = (int)p.grid.x;
+    pa.gy = (int)p.grid.y;
+    pa.gx = (int)p.grid.z;
+    if (std::is_same<P, PF32>::value) {
+        // one tile per resident block where that keeps most of them busy, else the launch's tiles
+        const long chunks = p.kf.flat_chunks;
+        const long parts = std::min((long)p.kf.nx, p.persist_blocks / chunks);
+        pa.planes = 2 * parts * chunks > p.persist_blocks ? (int)((p.kf.nx + parts - 1) / parts) : p.kf.XC;
+        pa.gz = (int)chunks;
+        pa.gy = 1;
+        pa.gx = (p.kf.nx + pa.planes - 1) / pa.planes;
+    }
+    const int blocks = std::min(pa.gz * pa.gy * pa.gx, p.persist_blocks);
     // the barrier counter and, 8 bytes on, the ticket counter
     cudaError_t e = cudaMemsetAsync(p.persist_bar, 0, 16, st);
     if (e == cudaSuccess) {
         GridK gk = p.kf;
         void *args[] = {&gk, &pa};
-        e = cudaLaunchCooperativeKernel(fn, dim3(blocks), p.block, args, 0, st);
+        e = cudaLaunchCooperativeKernel(fn, dim3(blocks), block, args, 0, st);
     }
     if (e != cudaSuccess) {
         set_last_cuda_error((int)e);

@@ -4,15 +4,17 @@
 // A grid of a few million cells takes tens of microseconds per half step, so
 // a run of two launches per step (plus detector gathers) is bound by launch
 // latency and by the partly filled last wave of each launch rather than by
-// memory.  Here the blocks share out the register-streaming tiles of a
-// half step (tile_update_E / tile_update_H, the same per-cell arithmetic as
-// the one-launch-per-half-step plan, so the same bits), then all blocks meet
-// at a grid-wide barrier before the other half step.  Detector gathers and
+// memory.  Here the blocks share out the flat (float32) or register-streaming
+// tiles of a half step (the same per-cell arithmetic as the plan with one
+// launch per half step, so the same bits), then all blocks meet at a grid-wide
+// barrier before the other half step.  Detector gathers and
 // DFT accumulation of a half step run after its barrier, interleaved with the
 // next half step (which never writes the field they read).
 //
-// Fields the other half step wrote are read with L2-only loads (the
-// read-only path may keep lines in L1 across the barrier).
+// Fields the other half step wrote are read with L2-only loads in the
+// register-streaming tiles and with ordinary loads in the flat ones (each
+// block's barrier ends in an acquire at GPU scope, which orders them); never
+// through the read-only path, which may keep lines in L1 across the barrier.
 //
 // The launch is cooperative (all blocks resident at once, so the barrier
 // cannot wait for a block that never runs).  Barrier waits are bounded: a
@@ -20,6 +22,7 @@
 // so do the others when their own waits expire; the context stays usable.
 #pragma once
 
+#include "fdtd_flat.cuh"
 #include "fdtd_kernels.cuh"
 
 namespace fdtd {
@@ -31,7 +34,8 @@ struct PersistArgs {
     long long n_steps;
     const double *wave;
     int n_columns;
-    int gz, gy, gx;  // register-streaming tile grid
+    int gz, gy, gx;     // register-streaming tile grid; flat: gz chunks of the plane, gx x chunks
+    int planes;         // flat: planes per x chunk
     int n_probe;
     const int64_t *probe_cells;
     void *trace_E, *trace_H;  // first rows of this call
@@ -106,7 +110,9 @@ __device__ __forceinline__ void persist_dft(const GridK &g, const fdtd_dft_desc 
 // (h + 1) ntiles) and the counter never needs resetting.  A block draws its
 // next ticket before its current tile runs, hiding the atomic's latency.
 // With no more tiles than blocks nothing is drawn.
-template <bool IS_E, class P, int V>
+// V: cells per thread of the register-streaming tiles, or 0 for flat tiles;
+// MAT: how the half step's material is read.
+template <bool IS_E, class P, int V, int MAT>
 __device__ __forceinline__ void persist_half(const GridK &g, const PersistArgs &a, const double *wave, int ntiles,
                                              unsigned long long base) {
     __shared__ int ticket_s;
@@ -119,8 +125,14 @@ __device__ __forceinline__ void persist_half(const GridK &g, const PersistArgs &
         if (lead && draw) next = atomicAdd(a.tickets, 1ull);
         const int tile = a.order ? a.order[t] : t;
         const int bx = tile % a.gz, by = (tile / a.gz) % a.gy, bz = tile / (a.gz * a.gy);
-        if constexpr (IS_E) tile_update_E<P, V, true>(g, wave, bx, by, bz, tile);
-        else tile_update_H<P, V, true>(g, wave, bx, by, bz, tile);
+        if constexpr (V == 0) {
+            const int xa = bz * a.planes;
+            flat_tile<P, IS_E, MAT>(g, wave, (unsigned)bx, xa, min(g.nx, xa + a.planes));
+        } else if constexpr (IS_E) {
+            tile_update_E<P, V, true, MAT>(g, wave, bx, by, bz, tile);
+        } else {
+            tile_update_H<P, V, true, MAT>(g, wave, bx, by, bz, tile);
+        }
         if (!draw) break;
         __syncthreads();  // every thread has read ticket_s
         if (lead) ticket_s = nblk + (int)(next - base);
@@ -129,8 +141,11 @@ __device__ __forceinline__ void persist_half(const GridK &g, const PersistArgs &
     }
 }
 
-template <class P, int V>
-__global__ void __launch_bounds__(kThreads) k_run_persistent(const GridK g, const PersistArgs a) {
+// Flat tiles: three blocks of 80 registers (with four of 64 the two inlined
+// tiles spill 500 bytes).
+template <class P, int V, int MAT_E, int MAT_H>
+__global__ void __launch_bounds__(kThreads, V == 0 ? 3 : (V == 1 ? 1 : 2))
+    k_run_persistent(const __grid_constant__ GridK g, const __grid_constant__ PersistArgs a) {
     using T = typename P::T;
     const int ntiles = a.gz * a.gy * a.gx;
     const long nthr = (long)gridDim.x * kThreads;
@@ -140,7 +155,7 @@ __global__ void __launch_bounds__(kThreads) k_run_persistent(const GridK g, cons
     unsigned epoch = 0;
     for (long long s = 0; s < a.n_steps; ++s) {
         const double *wave = a.n_columns > 0 ? a.wave + s * a.n_columns : nullptr;
-        persist_half<true, P, V>(g, a, wave, ntiles, base);
+        persist_half<true, P, V, MAT_E>(g, a, wave, ntiles, base);
         base += per_half;
         if (!grid_barrier(a.barrier, ++epoch, a.limit, g.status)) return;
         // E is final for this step: gathers and DFT overlap the H half
@@ -150,7 +165,7 @@ __global__ void __launch_bounds__(kThreads) k_run_persistent(const GridK g, cons
         }
         for (int d = 0; d < a.n_dft; ++d)
             persist_dft<T, P::COMP>(g, a.dft[d], a.phase + s * 2 * a.n_phase_columns, tid, nthr);
-        persist_half<false, P, V>(g, a, wave, ntiles, base);
+        persist_half<false, P, V, MAT_H>(g, a, wave, ntiles, base);
         base += per_half;
         if (!grid_barrier(a.barrier, ++epoch, a.limit, g.status)) return;
         if (a.n_probe) {

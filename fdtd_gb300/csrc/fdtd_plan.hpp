@@ -32,9 +32,12 @@ struct Plan {
     GridK kfH;         // the same for the H pass of staged plans (its own ring depth and stage layout)
     int pml_split;     // 1: PML slabs from fused_slabs on run as EPI_PML kernels after the fused pass
     int fused_slabs;   // with pml_split: leading slabs (normal to x or y) kept in the fused pass
-    int V;             // cells per thread along z
+    int V;             // cells per thread along z (flat: 1)
     dim3 grid, block;  // fused-pass launch shape
-    int variant;       // 1 register streaming, 2 TMA-staged
+    int variant;       // 1 flat or register streaming, 2 TMA-staged
+    int flat;          // variant 1 runs the flat half steps: float32 but the interior of a partition
+    int flat_general;  // flat half steps in their general form: PML slabs of one axis share cells, or
+                       // auxiliaries not aligned to a pair
     size_t smem_bytes; // dynamic shared memory of the TMA-staged kernels
     CUtensorMap maps[MAP_COUNT];
     const void *index_E, *index_H;  // one-byte material indices (MAT_IDS)
