@@ -1,6 +1,7 @@
 // Launch sequence of the reverse-time adjoint (fdtd_adjoint_run), float32 and
 // float64 instantiations.
 #include "fdtd_adjoint.cuh"
+#include "fdtd_adjoint_flat.cuh"
 #include "fdtd_adjoint_tma.cuh"
 #include "fdtd_launch.cuh"
 #include "fdtd_plan.hpp"
@@ -142,6 +143,27 @@ static void launch_adj_slab(const GridK &g, const AdjAux &x, int slab, long cell
     else launch_adj_slab_axis<T, IS_E, 2>(g, x, slab, cells, st);
 }
 
+template <bool TH, int MAT>
+static void adj_flat_mat(const Plan &p, const GridK &g, const AdjFlat &x, cudaStream_t st) {
+    k_adj_flat<float, TH, MAT><<<p.adj_flat_blocks, kFlatBlock, 0, st>>>(g, x);
+}
+
+// One flat transposed half step: the layers' current and next auxiliaries by
+// axis and side.
+template <bool TH>
+static void adj_flat(const Plan &p, const GridK &g, const AdjAux &aux, cudaStream_t st) {
+    AdjFlat x{};
+    for (int s = 0; s < g.nslab; ++s) {
+        const SlabK &S = g.slab[s];
+        x.old[S.axis][S.high] = TH ? aux.Ho[s] : aux.Eo[s];
+        x.now[S.axis][S.high] = TH ? aux.Hn[s] : aux.En[s];
+    }
+    const int mat = TH ? g.mat_H : g.mat_E;
+    if (mat == MAT_UNIFORM) adj_flat_mat<TH, MAT_UNIFORM>(p, g, x, st);
+    else if (mat == MAT_IDS) adj_flat_mat<TH, MAT_IDS>(p, g, x, st);
+    else adj_flat_mat<TH, MAT_FULL>(p, g, x, st);
+}
+
 template <class T, int V>
 static int adjoint_impl(Plan &p, const fdtd_adjoint_args *a, cudaStream_t st) {
     GridK g = p.k;
@@ -193,6 +215,15 @@ static int adjoint_impl(Plan &p, const fdtd_adjoint_args *a, cudaStream_t st) {
         gs.ey = p.kf.ey;
         gs.ez = p.kf.ez;
     }
+    // flat: auxiliaries aligned to a pair (the plan checked the rest)
+    bool flat = p.adj_flat && !staged && sizeof(T) == 4;
+    for (int q = 0; q < p.k.nslab && flat; ++q)
+        for (int r = 0; r < 2; ++r)
+            if (((uintptr_t)a->aux_E[p.slab_boundary[q]][r] | (uintptr_t)a->aux_H[p.slab_boundary[q]][r]) % 8)
+                flat = false;
+    GridK gf = p.kadj;
+    gf.E = a->lam_E;
+    gf.H = a->lam_H;
     auto slab_cells = [&](const SlabK &S) {
         return (long)(S.axis == 0 ? S.th : g.nx) * (S.axis == 1 ? S.th : g.ny) * (S.axis == 2 ? S.th : g.nz);
     };
@@ -238,6 +269,8 @@ static int adjoint_impl(Plan &p, const fdtd_adjoint_args *a, cudaStream_t st) {
         } else if (p.n_shell) {
             k_adj_H<T, V><<<p.adjin_grid, p.adjin_block, 0, st>>>(gi, x);
             k_adj_shell_H<T, SV><<<shell_blocks, kThreads, 0, st>>>(g, p.shellk, x);
+        } else if (flat) {
+            adj_flat<true>(p, gf, x, st);
         } else {
             k_adj_H<T, V><<<p.adj_grid, p.adj_block, 0, st>>>(gb, x);
         }
@@ -282,6 +315,8 @@ static int adjoint_impl(Plan &p, const fdtd_adjoint_args *a, cudaStream_t st) {
         } else if (p.n_shell) {
             k_adj_E<T, V><<<p.adjin_grid, p.adjin_block, 0, st>>>(gi, x);
             k_adj_shell_E<T, SV><<<shell_blocks, kThreads, 0, st>>>(g, p.shellk, x);
+        } else if (flat) {
+            adj_flat<false>(p, gf, x, st);
         } else {
             k_adj_E<T, V><<<p.adj_grid, p.adj_block, 0, st>>>(gb, x);
         }

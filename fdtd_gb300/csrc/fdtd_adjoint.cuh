@@ -711,29 +711,4 @@ __global__ void k_adj_slab_inc(const GridK g, int s, T *aux) {
     }
 }
 
-// curl_H(H) on an object's box (fdtd/grid.py:54-76 differences), for the
-// gradient of the reverse pass: out[box cell][c].
-template <class T>
-__global__ void k_capture_curl(const GridK g, int item, T *out) {
-    const ItemK &o = g.items[item];
-    const int b0 = o.hi[0] - o.lo[0], b1 = o.hi[1] - o.lo[1], b2 = o.hi[2] - o.lo[2];
-    const long total = (long)b0 * b1 * b2;
-    const T *H = (const T *)g.H;
-    const long sx = 3L * g.ny * g.nz, sy = 3L * g.nz;
-    for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < total; t += (long)gridDim.x * blockDim.x) {
-        const int i = o.lo[0] + (int)(t / ((long)b1 * b2)), j = o.lo[1] + (int)((t / b2) % b1),
-                  k = o.lo[2] + (int)(t % b2);
-        const T *h = H + 3 * (((size_t)i * g.ny + j) * g.nz + k);
-        const T dxHy = i > 0 ? h[1] - h[1 - sx] : T(0);
-        const T dxHz = i > 0 ? h[2] - h[2 - sx] : T(0);
-        const T dyHx = j > 0 ? h[0] - h[-sy] : T(0);
-        const T dyHz = j > 0 ? h[2] - h[2 - sy] : T(0);
-        const T dzHx = k > 0 ? h[0] - h[-3] : T(0);
-        const T dzHy = k > 0 ? h[1] - h[-2] : T(0);
-        out[3 * t] = dyHz - dzHy;
-        out[3 * t + 1] = dzHx - dxHz;
-        out[3 * t + 2] = dxHy - dyHx;
-    }
-}
-
 }  // namespace fdtd

@@ -1382,6 +1382,19 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
         p.kf.ez = ibox[5];
     }
     p.flat_general = flat && !flat_layers(p.kf, 2 * esize);
+    // the flat transposed half steps: float32 grids with every layer in the
+    // pass (the staged plans, split layers and partitions have their own)
+    p.kadj = p.k;
+    p.adj_flat = d->precision == FDTD_FLOAT32 && p.n_shell == 0 && p.pml_split == 0 &&
+                 flat_layers(p.kadj, 2 * esize);
+    if (p.adj_flat) {
+        const long chunks = ((long)d->ny * d->nz + kFlatBlock - 1) / kFlatBlock;
+        p.kadj.flat_chunks = (unsigned)chunks;
+        p.kadj.XC = flat_planes(d->nx, chunks, 4L * n_sm);
+        const long blocks = chunks * ((d->nx + p.kadj.XC - 1) / p.kadj.XC);
+        p.adj_flat = blocks < (1L << 31);
+        p.adj_flat_blocks = (unsigned)blocks;
+    }
     p.kfH = p.kf;
     if (p.variant == 2) {
         GridK *pass_k[2] = {&p.kf, &p.kfH};
@@ -1467,7 +1480,7 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
         // 64^3 1.25x, 192x192x96 1.07x
         const long auto_cells = d->precision == FDTD_FLOAT64 ? (8L << 20) : 3000000L;
         p.persistent = p.persist_ok && (d->persistent == 2 || (d->persistent == 0 && ncell < auto_cells));
-        p.persist_blocks = 0;
+        p.persist_blocks[0] = p.persist_blocks[1] = 0;
     }
     p.stats_ctas = std::max(1, std::min(4 * n_sm, FDTD_STATS_STATIC_MAX_ROWS));
     p.device = dev;

@@ -659,6 +659,37 @@ __global__ void k_dft(const T *__restrict__ E, const T *__restrict__ Elo, int ny
     }
 }
 
+// curl_H(H) of box cell t of an object (fdtd/grid.py:54-76 differences), for
+// the gradient of the reverse pass: out[t][c].
+template <class T>
+__device__ __forceinline__ void capture_curl(const GridK &g, const ItemK &o, const T *H, long t, T *out) {
+    const int b1 = o.hi[1] - o.lo[1], b2 = o.hi[2] - o.lo[2];
+    const long sx = 3L * g.ny * g.nz, sy = 3L * g.nz;
+    const int i = o.lo[0] + (int)(t / ((long)b1 * b2)), j = o.lo[1] + (int)((t / b2) % b1), k = o.lo[2] + (int)(t % b2);
+    const T *h = H + 3 * (((size_t)i * g.ny + j) * g.nz + k);
+    const T dxHy = i > 0 ? h[1] - h[1 - sx] : T(0);
+    const T dxHz = i > 0 ? h[2] - h[2 - sx] : T(0);
+    const T dyHx = j > 0 ? h[0] - h[-sy] : T(0);
+    const T dyHz = j > 0 ? h[2] - h[2 - sy] : T(0);
+    const T dzHx = k > 0 ? h[0] - h[-3] : T(0);
+    const T dzHy = k > 0 ? h[1] - h[-2] : T(0);
+    out[3 * t] = dyHz - dzHy;
+    out[3 * t + 1] = dzHx - dxHz;
+    out[3 * t + 2] = dxHy - dyHx;
+}
+
+__device__ __forceinline__ long item_cells(const ItemK &o) {
+    return (long)(o.hi[0] - o.lo[0]) * (o.hi[1] - o.lo[1]) * (o.hi[2] - o.lo[2]);
+}
+
+template <class T>
+__global__ void k_capture_curl(const GridK g, int item, T *out) {
+    const ItemK &o = g.items[item];
+    const long total = item_cells(o);
+    for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < total; t += (long)gridDim.x * blockDim.x)
+        capture_curl<T>(g, o, (const T *)g.H, t, out);
+}
+
 // Stand-alone curls, one thread per cell (fdtd/grid.py:29-76).
 template <class T>
 __global__ void k_curl_E(const T *__restrict__ E, T *out, int nx, int ny, int nz) {

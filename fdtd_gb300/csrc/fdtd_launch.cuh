@@ -308,21 +308,22 @@ static size_t stage_bytes_of(int tile_rows, int mat_E, int mat_H) {
 
 // The persistent loop over flat tiles for a plan's two material modes (an
 // indexed H material is read in full).
-template <class P>
+template <class P, bool CAP>
 static const void *persist_flat(int mat_E, int mat_H) {
     if (mat_H == MAT_UNIFORM) {
-        if (mat_E == MAT_UNIFORM) return (const void *)k_run_persistent<P, 0, MAT_UNIFORM, MAT_UNIFORM>;
-        if (mat_E == MAT_IDS) return (const void *)k_run_persistent<P, 0, MAT_IDS, MAT_UNIFORM>;
-        return (const void *)k_run_persistent<P, 0, MAT_FULL, MAT_UNIFORM>;
+        if (mat_E == MAT_UNIFORM) return (const void *)k_run_persistent<P, 0, MAT_UNIFORM, MAT_UNIFORM, CAP>;
+        if (mat_E == MAT_IDS) return (const void *)k_run_persistent<P, 0, MAT_IDS, MAT_UNIFORM, CAP>;
+        return (const void *)k_run_persistent<P, 0, MAT_FULL, MAT_UNIFORM, CAP>;
     }
-    if (mat_E == MAT_UNIFORM) return (const void *)k_run_persistent<P, 0, MAT_UNIFORM, MAT_FULL>;
-    if (mat_E == MAT_IDS) return (const void *)k_run_persistent<P, 0, MAT_IDS, MAT_FULL>;
-    return (const void *)k_run_persistent<P, 0, MAT_FULL, MAT_FULL>;
+    if (mat_E == MAT_UNIFORM) return (const void *)k_run_persistent<P, 0, MAT_UNIFORM, MAT_FULL, CAP>;
+    if (mat_E == MAT_IDS) return (const void *)k_run_persistent<P, 0, MAT_IDS, MAT_FULL, CAP>;
+    return (const void *)k_run_persistent<P, 0, MAT_FULL, MAT_FULL, CAP>;
 }
 
 // All steps of a call in one cooperative launch (fdtd_persistent.cuh).
 template <class P>
-static int run_persistent(Plan &p, const fdtd_run_args *a, bool detect, cudaStream_t st) {
+static int run_persistent(Plan &p, const fdtd_run_args *a, const fdtd_capture_args *cap, bool detect,
+                          cudaStream_t st) {
     PersistArgs pa{};
     pa.n_steps = a->n_steps;
     pa.wave = a->wave;
@@ -337,6 +338,11 @@ static int run_persistent(Plan &p, const fdtd_run_args *a, bool detect, cudaStre
     pa.n_phase_columns = p.n_phase_columns;
     pa.n_dft = detect ? (int)p.dft.size() : 0;
     for (int q = 0; q < pa.n_dft; ++q) pa.dft[q] = p.dft[q];
+    for (int q = 0; cap != nullptr && q < cap->n_curl; ++q) {
+        if (cap->curl[q] == nullptr) continue;
+        pa.curl_item[pa.n_curl] = q;
+        pa.curl[pa.n_curl++] = cap->curl[q];
+    }
     pa.barrier = p.persist_bar;
     pa.tickets = p.persist_tickets;
     pa.order = p.persist_order;
@@ -344,7 +350,8 @@ static int run_persistent(Plan &p, const fdtd_run_args *a, bool detect, cudaStre
     const void *fn = nullptr;
     dim3 block = p.block;
     if constexpr (std::is_same<P, PF32>::value) {
-        fn = persist_flat<P>(p.kf.mat_E, p.kf.mat_H);
+        fn = pa.n_curl ? persist_flat<P, true>(p.kf.mat_E, p.kf.mat_H)
+                       : persist_flat<P, false>(p.kf.mat_E, p.kf.mat_H);
         block = dim3(kFlatBlock);
     } else if (p.kf.mat_H == MAT_UNIFORM) {
         fn = p.V > 1 ? (const void *)k_run_persistent<P, P::V, MAT_FULL, MAT_UNIFORM>
@@ -353,7 +360,8 @@ static int run_persistent(Plan &p, const fdtd_run_args *a, bool detect, cudaStre
         fn = p.V > 1 ? (const void *)k_run_persistent<P, P::V, MAT_FULL, MAT_FULL>
                      : (const void *)k_run_persistent<P, 1, MAT_FULL, MAT_FULL>;
     }
-    if (p.persist_blocks == 0) {
+    int &resident = p.persist_blocks[pa.n_curl ? 1 : 0];
+    if (resident == 0) {
         int per_sm = 0, dev = 0, n_sm = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
@@ -362,7 +370,7 @@ static int run_persistent(Plan &p, const fdtd_run_args *a, bool detect, cudaStre
             set_last_cuda_error((int)e);
             return FDTD_ERR_CUDA;
         }
-        p.persist_blocks = per_sm * n_sm;
+        resident = per_sm * n_sm;
     }
     pa.gz = (int)p.grid.x;
     pa.gy = (int)p.grid.y;
@@ -370,13 +378,13 @@ static int run_persistent(Plan &p, const fdtd_run_args *a, bool detect, cudaStre
     if (std::is_same<P, PF32>::value) {
         // one tile per resident block where that keeps most of them busy, else the launch's tiles
         const long chunks = p.kf.flat_chunks;
-        const long parts = std::min((long)p.kf.nx, p.persist_blocks / chunks);
-        pa.planes = 2 * parts * chunks > p.persist_blocks ? (int)((p.kf.nx + parts - 1) / parts) : p.kf.XC;
+        const long parts = std::min((long)p.kf.nx, resident / chunks);
+        pa.planes = 2 * parts * chunks > resident ? (int)((p.kf.nx + parts - 1) / parts) : p.kf.XC;
         pa.gz = (int)chunks;
         pa.gy = 1;
         pa.gx = (p.kf.nx + pa.planes - 1) / pa.planes;
     }
-    const int blocks = std::min(pa.gz * pa.gy * pa.gx, p.persist_blocks);
+    const int blocks = std::min(pa.gz * pa.gy * pa.gx, resident);
     // the barrier counter and, 8 bytes on, the ticket counter
     cudaError_t e = cudaMemsetAsync(p.persist_bar, 0, 16, st);
     if (e == cudaSuccess) {
@@ -425,8 +433,10 @@ static int run_impl(Plan &p, const fdtd_run_args *a, const fdtd_capture_args *ca
     const GridK &g = p.k;
     const int pblocks = (3 * p.n_probe + kThreads - 1) / kThreads;
     // small plans: every full step of the call in one cooperative launch
-    if (p.persistent && a->half == 0 && cap == nullptr && a->n_steps >= 2)
-        return run_persistent<P>(p, a, detect, st);
+    int captures = 0;
+    for (int q = 0; cap != nullptr && q < cap->n_curl; ++q) captures += cap->curl[q] != nullptr;
+    if (p.persistent && a->half == 0 && captures <= (p.flat ? kPersistMaxCurl : 0) && a->n_steps >= 2)
+        return run_persistent<P>(p, a, cap, detect, st);
     // one pass per full step (float32 plans that have it), in pairs: the first
     // pass of a pair writes the alternate buffers, the second the caller's; an
     // odd last step runs the two passes

@@ -28,6 +28,7 @@
 namespace fdtd {
 
 constexpr int kPersistMaxDft = 4;
+constexpr int kPersistMaxCurl = 4;
 
 // Everything the persistent loop needs besides the GridK.
 struct PersistArgs {
@@ -43,6 +44,9 @@ struct PersistArgs {
     int n_phase_columns;
     int n_dft;
     fdtd_dft_desc dft[kPersistMaxDft];
+    int n_curl;                       // object boxes whose curl of H each step keeps
+    int curl_item[kPersistMaxCurl];
+    void *curl[kPersistMaxCurl];      // n_steps rows of 3 values per box cell
     unsigned *barrier;                // arrival counter, zero at launch
     unsigned long long *tickets;      // tile tickets drawn, zero at launch
     const int *order;                 // tile of each ticket, heaviest first (null: grid order)
@@ -101,6 +105,17 @@ __device__ __forceinline__ void persist_dft(const GridK &g, const fdtd_dft_desc 
     }
 }
 
+// The object boxes' curls of step s.
+template <class T>
+__device__ __forceinline__ void persist_capture(const GridK &g, const PersistArgs &a, long long s, long tid, long nthr) {
+    for (int c = 0; c < a.n_curl; ++c) {
+        const ItemK &o = g.items[a.curl_item[c]];
+        const long cells = item_cells(o);
+        for (long q = tid; q < cells; q += nthr)
+            capture_curl<T>(g, o, (const T *)g.H, q, (T *)a.curl[c] + s * 3 * cells);
+    }
+}
+
 // The tiles of one half step: each block's first tile is its own (the
 // heaviest tiles go to the first blocks), the rest are handed out by ticket:
 // a block draws tickets from one counter until it draws one past the last
@@ -143,7 +158,9 @@ __device__ __forceinline__ void persist_half(const GridK &g, const PersistArgs &
 
 // Flat tiles: three blocks of 80 registers (with four of 64 the two inlined
 // tiles spill 500 bytes).
-template <class P, int V, int MAT_E, int MAT_H>
+// CAP: steps that keep the curls of object boxes, apart from the plain run,
+// whose tiles would lose the registers (128^3: 52.9 -> 56.2 us per step).
+template <class P, int V, int MAT_E, int MAT_H, bool CAP = false>
 __global__ void __launch_bounds__(kThreads, V == 0 ? 3 : (V == 1 ? 1 : 2))
     k_run_persistent(const __grid_constant__ GridK g, const __grid_constant__ PersistArgs a) {
     using T = typename P::T;
@@ -155,6 +172,8 @@ __global__ void __launch_bounds__(kThreads, V == 0 ? 3 : (V == 1 ? 1 : 2))
     unsigned epoch = 0;
     for (long long s = 0; s < a.n_steps; ++s) {
         const double *wave = a.n_columns > 0 ? a.wave + s * a.n_columns : nullptr;
+        // (H is final: captures run beside the E half)
+        if constexpr (CAP) persist_capture<T>(g, a, s, tid, nthr);
         persist_half<true, P, V, MAT_E>(g, a, wave, ntiles, base);
         base += per_half;
         if (!grid_barrier(a.barrier, ++epoch, a.limit, g.status)) return;

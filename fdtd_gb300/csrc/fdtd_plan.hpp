@@ -62,6 +62,9 @@ struct Plan {
     int adj_V;
     dim3 adj_grid, adj_block;
     int adj_TZ, adj_TY, adj_XC;
+    int adj_flat;      // the flat transposed half steps (fdtd_adjoint_flat.cuh): float32, layers in the pass
+    GridK kadj;        // their GridK (kadj.E, kadj.H: set per call)
+    unsigned adj_flat_blocks;
     // partition plans: the transposed passes' tiling of the interior box
     dim3 adjin_grid, adjin_block;
     int adjin_TZ, adjin_TY, adjin_XC;
@@ -83,7 +86,7 @@ struct Plan {
     unsigned *persist_bar;
     unsigned long long *persist_tickets;
     const int *persist_order;
-    int persist_blocks;
+    int persist_blocks[2];  // of the plain kernel and of the one that captures curls
     // interior/shell partition (pml_mode 4): the fused pass's tiles cover the
     // interior box; the n_shell boxes around it run one thread per cell with
     // every slab (kshell: the plan's GridK with per-block lists)
