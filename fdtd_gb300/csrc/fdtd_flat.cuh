@@ -314,56 +314,110 @@ __device__ __forceinline__ void flat_source(const ItemK &s, int ny, int nz, cons
     }
 }
 
-// Planes [xa, xb) of a chunk of the plane.  A warp whose cells have all their
-// neighbours in the grid and lie in no layer and no object runs the short
-// loop, two planes loaded before the first is computed; the others run the
-// full one.
-template <class P, bool IS_E, int MAT>
-__device__ __forceinline__ void flat_tile(const GridK &g, const double *__restrict__ wave, unsigned chunk, int xa,
-                                          int xb) {
+// What a thread knows of its column of a tile before it marches.  A block of
+// the persistent loop that keeps its tile works it out once per launch.
+template <class T>
+struct FlatColumn {
+    FlatPair<T> *yq, *wq;  // the layers normal to y and z: pair of the march's first plane,
+    T yb, yc, wb, wc;      // coefficients,
+    int ystep, wstep;      // step to the next plane's pair
+    int j, k;
+    unsigned omask, smask;  // objects and sources whose y and z ranges hold the cell
+    int ob0, ob1;           // the chunk's objects in the lists (past 32 tested plane by plane)
+    int listed;             // sources in the chunk's list, applied after the march
+    bool in, yok, zok, special, yinc, winc;
+};
+
+template <class P, bool IS_E>
+__device__ __forceinline__ FlatColumn<typename P::T> flat_column(const GridK &g, unsigned chunk, int xa, int xb) {
     using T = typename P::T;
     constexpr int dir = IS_E ? 1 : -1;
-    const int nx = g.nx, ny = g.ny, nz = g.nz;
+    const int ny = g.ny, nz = g.nz;
     const FlatPlace pl = flat_place(g, chunk);
     const int j = pl.j, k = pl.k;
-    const long jk = (long)j * nz + k, nyz = (long)ny * nz;
-    const bool yok = IS_E ? j > 0 : j < ny - 1, zok = IS_E ? k > 0 : k < nz - 1;
-    // to the y and z neighbours (the cell itself where there is none)
-    const long oy = yok ? -dir * 3 * nz : 0, oz = zok ? -dir * 3 : 0;
+    FlatColumn<T> o;
+    o.in = pl.in;
+    o.j = j;
+    o.k = k;
+    o.yok = IS_E ? j > 0 : j < ny - 1;
+    o.zok = IS_E ? k > 0 : k < nz - 1;
     const int i0 = IS_E ? xa : xb - 1;
 
     // an object or source whose y and z ranges hold this cell sets a bit, so
     // that a plane tests only those
-    int ob0 = 0, ob1 = 0;
-    unsigned omask = 0, smask = 0;
+    o.ob0 = o.ob1 = 0;
+    o.omask = o.smask = 0;
     if constexpr (IS_E) {
-        ob0 = g.obj_off[chunk];
-        ob1 = g.obj_off[chunk + 1];
-        for (int it = ob0; it < min(ob1, ob0 + 32); ++it) {
-            const ItemK &o = g.items[g.obj_idx[it]];
-            if (o.lo[0] < xb && o.hi[0] > xa && j >= o.lo[1] && j < o.hi[1] && k >= o.lo[2] && k < o.hi[2])
-                omask |= 1u << (it - ob0);
+        o.ob0 = g.obj_off[chunk];
+        o.ob1 = g.obj_off[chunk + 1];
+        for (int it = o.ob0; it < min(o.ob1, o.ob0 + 32); ++it) {
+            const ItemK &b = g.items[g.obj_idx[it]];
+            if (b.lo[0] < xb && b.hi[0] > xa && j >= b.lo[1] && j < b.hi[1] && k >= b.lo[2] && k < b.hi[2])
+                o.omask |= 1u << (it - o.ob0);
         }
-        ob1 = max(ob1, ob0 + 32);  // (past 32 the rest is tested plane by plane)
+        o.ob1 = max(o.ob1, o.ob0 + 32);
     }
     const FlatSources &src = IS_E ? g.src_E : g.src_H;
-    int listed = 0;  // more sources than the parameters hold: the chunk's list, after the march
+    o.listed = 0;  // more sources than the parameters hold: the chunk's list
     if (src.n >= 0) {
 #pragma unroll
         for (int q = 0; q < kFlatSources; ++q)
             if (q < src.n && src.item[q].lo[0] < xb && src.item[q].hi[0] > xa && j >= src.item[q].lo[1] &&
                 j < src.item[q].hi[1] && k >= src.item[q].lo[2] && k < src.item[q].hi[2])
-                smask |= 1u << q;
+                o.smask |= 1u << q;
     } else {
         const int *off = IS_E ? g.srcE_off : g.srcH_off;
-        listed = off[chunk + 1] - off[chunk];
+        o.listed = off[chunk + 1] - off[chunk];
     }
     bool ylow, zlow;
     const int ly = flat_side(g.lay[1], j, ylow), lz = flat_side(g.lay[2], k, zlow);
-    const bool special =
-        __any_sync(0xffffffffu, pl.in && (!yok || (!zok && nz > 1) || ly >= 0 || lz >= 0 || omask != 0 || smask != 0 ||
-                                          ob1 > ob0 + 32));
-    if (!pl.in) return;
+    o.special =
+        __any_sync(0xffffffffu, pl.in && (!o.yok || (!o.zok && nz > 1) || ly >= 0 || lz >= 0 || o.omask != 0 ||
+                                          o.smask != 0 || o.ob1 > o.ob0 + 32));
+    FlatLayer<T> Y{nullptr, T(0), T(0), false}, W = Y;
+    o.ystep = o.wstep = 0;
+    if (pl.in && ly >= 0) {
+        const int th = ylow ? g.lay[1][0].th : g.lay[1][1].th;
+        Y = flat_layer_at<T, IS_E>(g.lay[1], ly, ylow, ((long)i0 * th + ly) * nz + k);
+        o.ystep = dir * th * nz;
+    }
+    if (pl.in && lz >= 0) {
+        const int thp = zlow ? g.lay[2][0].thp : g.lay[2][1].thp;
+        W = flat_layer_at<T, IS_E>(g.lay[2], lz, zlow, ((long)i0 * ny + j) * thp + lz);
+        o.wstep = dir * ny * thp;
+    }
+    o.yq = Y.q;
+    o.yb = Y.b;
+    o.yc = Y.c;
+    o.yinc = Y.inc;
+    o.wq = W.q;
+    o.wb = W.b;
+    o.wc = W.c;
+    o.winc = W.inc;
+    return o;
+}
+
+// Planes [xa, xb) of a column.  A warp whose cells have all their neighbours in
+// the grid and lie in no layer and no object runs the short loop, two planes
+// loaded before the first is computed; the others run the full one.
+template <class P, bool IS_E, int MAT>
+__device__ __forceinline__ void flat_march(const GridK &g, const double *__restrict__ wave, unsigned chunk, int xa,
+                                           int xb, const FlatColumn<typename P::T> &col) {
+    using T = typename P::T;
+    constexpr int dir = IS_E ? 1 : -1;
+    if (!col.in) return;
+    const int nx = g.nx, ny = g.ny, nz = g.nz;
+    const int j = col.j, k = col.k;
+    const long jk = (long)j * nz + k, nyz = (long)ny * nz;
+    const bool yok = col.yok, zok = col.zok, special = col.special;
+    // to the y and z neighbours (the cell itself where there is none)
+    const long oy = yok ? -dir * 3 * nz : 0, oz = zok ? -dir * 3 : 0;
+    const int i0 = IS_E ? xa : xb - 1;
+    const int ob0 = col.ob0, ob1 = col.ob1, listed = col.listed;
+    const unsigned omask = col.omask, smask = col.smask;
+    const FlatSources &src = IS_E ? g.src_E : g.src_H;
+    FlatLayer<T> X{nullptr, T(0), T(0), false}, Y{col.yq, col.yb, col.yc, col.yinc}, W{col.wq, col.wb, col.wc, col.winc};
+    const int ystep = col.ystep, wstep = col.wstep;
 
     const T courant = courant_of<T>(g);
     const T *lut = (const T *)(IS_E ? g.mlut_E : g.mlut_H);
@@ -385,21 +439,6 @@ __device__ __forceinline__ void flat_tile(const GridK &g, const double *__restri
     if (xok) {
         s.by = s.pn[1 - step];
         s.bz = s.pn[2 - step];
-    }
-
-    FlatLayer<T> X{nullptr, T(0), T(0), false}, Y{nullptr, T(0), T(0), false}, W{nullptr, T(0), T(0), false};
-    int ystep = 0, wstep = 0;  // to the next plane's pair
-    if (special) {
-        if (ly >= 0) {
-            const int th = ylow ? g.lay[1][0].th : g.lay[1][1].th;
-            Y = flat_layer_at<T, IS_E>(g.lay[1], ly, ylow, ((long)i0 * th + ly) * nz + k);
-            ystep = dir * th * nz;
-        }
-        if (lz >= 0) {
-            const int thp = zlow ? g.lay[2][0].thp : g.lay[2][1].thp;
-            W = flat_layer_at<T, IS_E>(g.lay[2], lz, zlow, ((long)i0 * ny + j) * thp + lz);
-            wstep = dir * ny * thp;
-        }
     }
 
     const int end = IS_E ? xb : xa - 1;  // the march stops before this plane
@@ -534,6 +573,12 @@ __device__ __forceinline__ void flat_tile(const GridK &g, const double *__restri
         flat_sources<P>(g, idx, listed, wave, xa, xb, j, k, jk, (T *)(IS_E ? g.E : g.H),
                         (T *)(IS_E ? g.Elo : g.Hlo));
     }
+}
+
+template <class P, bool IS_E, int MAT>
+__device__ __forceinline__ void flat_tile(const GridK &g, const double *__restrict__ wave, unsigned chunk, int xa,
+                                          int xb) {
+    flat_march<P, IS_E, MAT>(g, wave, chunk, xa, xb, flat_column<P, IS_E>(g, chunk, xa, xb));
 }
 
 // The same with the per-cell body of the staged passes, which takes layers of
