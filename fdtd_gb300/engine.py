@@ -149,17 +149,67 @@ _FUSION_REASONS = {
 }
 
 
+def _raw_stream():
+    """Handle of the current CUDA stream."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+
+
+class _Ring:
+    """Slots of one stream for small tables: pinned host and device memory of
+    the same layout.  A slot comes round again after every other one; the event
+    recorded when its half of the ring was left then has to have passed."""
+
+    SLOTS, WORDS = 64, 512
+
+    def __init__(self, device):
+        self.host = torch.empty((self.SLOTS, self.WORDS), dtype=torch.float64).pin_memory()
+        self.dev = torch.empty((self.SLOTS, self.WORDS), dtype=torch.float64, device=device)
+        self.flat = self.host.numpy()
+        self.host_slots, self.dev_slots = list(self.host.unbind(0)), list(self.dev.unbind(0))
+        self.left = [None, None]
+        self.turn = 0
+
+    def upload(self, array):
+        k = self.turn
+        self.turn = (k + 1) % self.SLOTS
+        half = self.SLOTS // 2
+        if k % half == 0:
+            h = k // half
+            ev = torch.cuda.Event()
+            ev.record()
+            self.left[1 - h] = ev
+            if self.left[h] is not None:
+                self.left[h].synchronize()
+        self.flat[k, :array.size] = array.reshape(-1)
+        dev = self.dev_slots[k]
+        dev.copy_(self.host_slots[k], non_blocking=True)
+        return dev
+
+
 class _PinnedStager:
-    """Double-buffered pinned host staging for small per-call tables."""
+    """Pinned host staging for per-call tables.  Small ones (a program that
+    steps call by call) go through a ring of the current stream, which
+    allocates nothing and waits for nothing per call; larger ones, and any
+    under stream capture, through two buffers that grow."""
+
+    MAX_RINGS = 4
 
     def __init__(self):
         self._bufs = [None, None]
         self._events = [None, None]
         self._dev = None
         self._turn = 0
+        self._rings = {}
 
     def upload(self, array, device):
         n = array.size
+        if n <= _Ring.WORDS and not torch.cuda.is_current_stream_capturing():
+            key = _raw_stream()
+            ring = self._rings.get(key)
+            if ring is None and len(self._rings) < self.MAX_RINGS:
+                ring = self._rings[key] = _Ring(device)
+            if ring is not None:
+                return ring.upload(array)
         k = self._turn
         self._turn ^= 1
         if self._events[k] is not None:
@@ -213,7 +263,7 @@ class Engine:
     # --- plan -------------------------------------------------------------------
     def _state_key(self):
         g = self.grid
-        return (tuple(o._coef_key() for o in g.objects), self.x_chunk, tuple(sorted(self.tuning.items())),
+        return (tuple(o._coef_key() for o in g.objects), self.x_chunk, tuple(self.tuning.values()),
                 g.courant_number, g._E.data_ptr(), g._H.data_ptr())
 
     def refresh(self):
@@ -695,7 +745,7 @@ class Engine:
                         det = src.current_detector
                         frozen = sum(c.shape[0] for c in det._frozen["I"])
                         src._note_steps(q0, n, frozen, self.rec_I - 1)
-        stream = ctypes.c_void_p(torch.cuda.current_stream(g._device).cuda_stream)
+        stream = ctypes.c_void_p(_raw_stream())
         if capture is None:
             _native.check(lib.fdtd_run(self.plan, ctypes.byref(a), stream), "fdtd_run")
         else:

@@ -256,6 +256,10 @@ class Grid:
             self._engine.refresh()
         return self._engine
 
+    def _stepper(self):
+        """The engine for a call that refreshes it itself (run, half)."""
+        return self._engine if self._engine is not None else self._ensure_engine()
+
     def run(self, total_time, progress_bar: bool = True):
         """Run ``total_time`` steps (int) or seconds (float)."""
         if isinstance(total_time, float):
@@ -263,7 +267,7 @@ class Grid:
         n = int(total_time)
         if n <= 0:
             return
-        eng = self._ensure_engine()
+        eng = self._stepper()
         bar = None
         if progress_bar:
             try:
@@ -288,15 +292,15 @@ class Grid:
 
     def step(self):
         """One E half step, one H half step, then time_steps_passed += 1."""
-        self._ensure_engine().run(1)
+        self._stepper().run(1)
 
     def update_E(self):
         """The E half step at the current time_steps_passed (no increment)."""
-        self._ensure_engine().half("E")
+        self._stepper().half("E")
 
     def update_H(self):
         """The H half step at the current time_steps_passed (no increment)."""
-        self._ensure_engine().half("H")
+        self._stepper().half("H")
 
     def reset(self):
         """Zero E and H and the step counter (PML auxiliaries are kept, like
