@@ -164,6 +164,20 @@ static void adj_flat(const Plan &p, const GridK &g, const AdjAux &aux, cudaStrea
     else adj_flat_mat<TH, MAT_FULL>(p, g, x, st);
 }
 
+// The transposed shell kernels of a partition.
+template <class T, bool TH>
+static void adj_shell(const Plan &p, const GridK &g, const AdjAux &x, unsigned blocks, cudaStream_t st) {
+    if constexpr (sizeof(T) == 4) {
+        if (p.shell_v == 2) {
+            if (TH) k_adj_shell_H<T, 2><<<blocks, kThreads, 0, st>>>(g, p.shellk, x);
+            else k_adj_shell_E<T, 2><<<blocks, kThreads, 0, st>>>(g, p.shellk, x);
+            return;
+        }
+    }
+    if (TH) k_adj_shell_H<T, 1><<<blocks, kThreads, 0, st>>>(g, p.shellk, x);
+    else k_adj_shell_E<T, 1><<<blocks, kThreads, 0, st>>>(g, p.shellk, x);
+}
+
 template <class T, int V>
 static int adjoint_impl(Plan &p, const fdtd_adjoint_args *a, cudaStream_t st) {
     GridK g = p.k;
@@ -195,7 +209,6 @@ static int adjoint_impl(Plan &p, const fdtd_adjoint_args *a, cudaStream_t st) {
         gi.ey = p.kf.ey;
         gi.ez = p.kf.ez;
     }
-    constexpr int SV = shell_v<T>();
     const unsigned shell_blocks = p.n_shell ? p.shellk.first[p.shellk.nbox] : 0u;
     // staged forward plans with the slabs on their own, or staged partition
     // interiors: staged transposed passes (over the interior box, then the
@@ -265,12 +278,12 @@ static int adjoint_impl(Plan &p, const fdtd_adjoint_args *a, cudaStream_t st) {
         if (staged) {
             const int rc = adj_staged<T>(p, gs, true, st);
             if (rc != FDTD_OK) return rc;
-            if (p.n_shell) k_adj_shell_H<T, SV><<<shell_blocks, kThreads, 0, st>>>(g, p.shellk, x);
-        } else if (p.n_shell) {
-            k_adj_H<T, V><<<p.adjin_grid, p.adjin_block, 0, st>>>(gi, x);
-            k_adj_shell_H<T, SV><<<shell_blocks, kThreads, 0, st>>>(g, p.shellk, x);
+            if (p.n_shell) adj_shell<T, true>(p, g, x, shell_blocks, st);
         } else if (flat) {
             adj_flat<true>(p, gf, x, st);
+        } else if (p.n_shell) {
+            k_adj_H<T, V><<<p.adjin_grid, p.adjin_block, 0, st>>>(gi, x);
+            adj_shell<T, true>(p, g, x, shell_blocks, st);
         } else {
             k_adj_H<T, V><<<p.adj_grid, p.adj_block, 0, st>>>(gb, x);
         }
@@ -311,12 +324,12 @@ static int adjoint_impl(Plan &p, const fdtd_adjoint_args *a, cudaStream_t st) {
         if (staged) {
             const int rc = adj_staged<T>(p, gs, false, st);
             if (rc != FDTD_OK) return rc;
-            if (p.n_shell) k_adj_shell_E<T, SV><<<shell_blocks, kThreads, 0, st>>>(g, p.shellk, x);
-        } else if (p.n_shell) {
-            k_adj_E<T, V><<<p.adjin_grid, p.adjin_block, 0, st>>>(gi, x);
-            k_adj_shell_E<T, SV><<<shell_blocks, kThreads, 0, st>>>(g, p.shellk, x);
+            if (p.n_shell) adj_shell<T, false>(p, g, x, shell_blocks, st);
         } else if (flat) {
             adj_flat<false>(p, gf, x, st);
+        } else if (p.n_shell) {
+            k_adj_E<T, V><<<p.adjin_grid, p.adjin_block, 0, st>>>(gi, x);
+            adj_shell<T, false>(p, g, x, shell_blocks, st);
         } else {
             k_adj_E<T, V><<<p.adj_grid, p.adj_block, 0, st>>>(gb, x);
         }

@@ -32,6 +32,10 @@ static int next_pow2(int v) {
 }
 
 static bool aligned16(const void *ptr) { return ((uintptr_t)ptr & 15u) == 0; }
+static bool aligned8(const void *ptr) { return ((uintptr_t)ptr & 7u) == 0; }
+
+// Cells from which a thick shell is split off automatically (see mode 4 below).
+static const long kPartition32 = 3800000, kPartition32odd = 2600000, kPartition64 = 500000, kPartition32c = 800000;
 
 // Threads along z of a register-streaming tile for zt threads' worth of
 // cells: the next power of two up to 32, or 16 where that pads less (config 5,
@@ -366,12 +370,27 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
     // written once per half step (the split slab kernels re-read each slab
     // cell the bulk pass has just written), and each cell still gets bulk,
     // objects, slabs in registration order and sources in that order, as in
-    // every mode.  Automatic on grids of 8M cells or more whose shell holds
-    // at least a fifth of the cells, a tenth in float64 (float32 ms per step, split slabs vs
-    // partition: config 2 0.443 vs 0.375, config 5 0.618 vs 0.608; float64
-    // config 2 1.74 vs 1.49; float32c config 5 1.10 vs 0.85; config 3, 12 %
-    // of its cells in the shell, stays faster with its slabs split: 5.47 vs
-    // 5.77 float32).
+    // every mode.  Automatic where the shell holds at least a fifth of the
+    // cells, a tenth in float64 and where rows do not divide into vectors
+    // (config 3, 12 % of its cells in the shell, stays faster with its slabs
+    // split in float32: 5.47 vs 5.77 ms per step; 377x257x277 float32, 19 %,
+    // fused 666, partition 524 us), on grids from 3.8M cells in float32 (2.6M
+    // where rows do not divide), 0.5M in float64 and 0.8M in float32c, whose
+    // shell cells otherwise hold up the warps or the FP64 pipe for the few
+    // lanes that have one.  us per step, fused vs partition: float32 (flat
+    // tiles) 1.9M cells 57.5 vs 60.6, 3.5M 107 vs 110, 4.1M 127 vs 116, 5.1M
+    // 157 vs 135, 6.9M 187 vs 171, 20M 505 vs 442, odd rows 2.7M 105 vs 106,
+    // 2.9M 114 vs 91; float64 (register tiles) 0.26M 58 vs 68, 0.6M 107 vs 97,
+    // 1.1M 209 vs 159, 2.1M 300 vs 255, 5.1M 524 vs 491, 6.9M 770 vs 628;
+    // float32c 0.26M 20 vs 31, 1.1M 70 vs 58, 1.9M 104 vs 82, 5.7M 225 vs 186,
+    // 30M odd rows, 10 %, 902 vs 822.
+    // cells per shell thread along z: two floats where rows are even, else one
+    p.shell_v = d->precision == FDTD_FLOAT64 || d->nz % 2 != 0 || !aligned8(d->E) || !aligned8(d->H) ||
+                        !aligned8(d->inv_eps) || !aligned8(d->inv_mu) ||
+                        (comp && (!aligned8(d->E_lo) || !aligned8(d->H_lo)))
+                    ? 1 : 2;
+    for (int s = 0; s < g.nslab; ++s)
+        if (!aligned16(g.slab[s].psiE) || !aligned16(g.slab[s].psiH)) p.shell_v = 1;
     int ibox[6] = {0, 0, 0, d->nx, d->ny, d->nz};  // tile box of the fused pass: [lo, hi) per axis
     p.n_shell = 0;
     p.shell_overlap = 0;
@@ -390,22 +409,25 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
         // interior from z = 20); float64 on 4-cell boundaries (96 bytes; the
         // field maps' x coordinate, 3 k esize / 8, is then even; config 5
         // float64 2.42 vs 2.47 ms with 12 fewer shell cells per z face)
-        const bool stg = d->variant == 2 || (d->variant == 0 && d->precision == FDTD_FLOAT32 &&
-                                              mat_want[0] != MAT_FULL && mat_want[1] != MAT_FULL);
-        const bool idx = stg && (mat_want[0] == MAT_IDS || mat_want[1] == MAT_IDS);
-        const int za = idx || d->precision != FDTD_FLOAT64 ? 16 : 4;
+        // Rows that do not divide into vectors (an odd nz, say) leave the
+        // interior to one cell per thread, and their z faces need no alignment
+        // but the shell threads' own.
+        const int za = !vec ? p.shell_v : (d->precision != FDTD_FLOAT64 ? 16 : 4);
+        const int zu = vec ? vmax : p.shell_v;
         lo[2] = (lo[2] + za - 1) / za * za;
-        hi[2] = hi[2] / vmax * vmax;
+        hi[2] = hi[2] / zu * zu;
         const bool inner = lo[0] < hi[0] && lo[1] < hi[1] && lo[2] < hi[2];
-        const bool ok = g.nslab > 0 && !slab_after_periodic && vec && inner;
-        if (pml_base == 4 && !ok) return FDTD_ERR_UNSUPPORTED;
+        const bool ok = g.nslab > 0 && !slab_after_periodic && (vec || d->nz > 1) && inner;
+        if (pml_base == 4 && !(ok && vec)) return FDTD_ERR_UNSUPPORTED;
         bool want = ok && pml_base == 4;
-        if (ok && pml_base == 0 && ncell >= (8L << 20)) {
-            // a fifth of the cells in the shell; float64 (arithmetic bound,
-            // register-streaming interior) from a tenth (config 3: 29.1 vs
-            // 30.4 ms per step)
+        const long from = d->precision == FDTD_FLOAT64 ? kPartition64
+                          : d->precision == FDTD_FLOAT32C ? kPartition32c
+                          : vec                           ? kPartition32 : kPartition32odd;
+        if (ok && pml_base == 0 && d->persistent != 2 && ncell >= from) {
+            // float64 (arithmetic bound, register-streaming interior) from a
+            // tenth: config 3 29.1 vs 30.4 ms per step
             const long inside = (long)(hi[0] - lo[0]) * (hi[1] - lo[1]) * (hi[2] - lo[2]);
-            const long frac = d->precision == FDTD_FLOAT64 ? 10 : 5;
+            const long frac = d->precision == FDTD_FLOAT64 || !vec ? 10 : 5;
             want = frac * (ncell - inside) >= ncell;
         }
         if (want) {
@@ -487,11 +509,14 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
     bool fused_z = false;  // a z slab inside the fused pass (divergent warps)
     for (int s = 0; s < ks; ++s) fused_z |= g.slab[s].axis == 2;
     // a partition's interior: the staged pass for float32 with compact
-    // materials on both passes, else the register-streaming one (measured:
-    // config 2, full permittivity, 0.375 vs 0.494 ms per step; config 5
-    // float64 2.49 vs 2.57, float32c 0.85 vs 0.95; float32 config 5 with
-    // compact materials 0.608 vs 0.636)
-    const bool shell_tma = d->precision == FDTD_FLOAT32 && mat_want[0] != MAT_FULL && mat_want[1] != MAT_FULL;
+    // materials on both passes from 24M cells, else the register-streaming one
+    // (config 2, full permittivity, 0.375 vs 0.494 ms per step; config 5
+    // float64 2.49 vs 2.57, float32c 0.85 vs 0.95; float32 with compact
+    // materials, staged vs register, us per step: 16.8M cells 413 vs 370,
+    // 18.5M 410 vs 373, 24.2M 518 vs 491, 24.6M 466 vs 482, 28M 558 vs 582,
+    // 64M 1072 vs 1166, 87M 1582 vs 1658)
+    const bool shell_tma = d->precision == FDTD_FLOAT32 && mat_want[0] != MAT_FULL && mat_want[1] != MAT_FULL &&
+                           ncell >= 24000000;
     const bool tma = d->variant == 2 || (d->variant == 0 && vec && !fused_z && (long)bnz * 3 * (long)esize >= 768 &&
                                          (p.n_shell == 0 || shell_tma));
     Tiling t{};
@@ -651,7 +676,16 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
     g.nlut_H = g.mat_H == MAT_FULL ? 0 : d->n_mu_table;
     g.mid_E = g.mat_E == MAT_IDS ? d->eps_index : nullptr;
     g.mid_H = g.mat_H == MAT_IDS ? d->mu_index : nullptr;
-    const bool flat = !use_tma && d->precision == FDTD_FLOAT32 && p.n_shell == 0;
+    // Flat half steps for float32, but for large 2D grids of several materials
+    // (few cells of a plane are in layers there, and the 40 registers of the
+    // register tiles keep more warps on the loads).  us per step, flat vs
+    // register: 1186x3541 one material 94 vs 99, blocks 120 vs 106, with an
+    // object 121 vs 106; 3000^2 219 vs 205; in the persistent loop with an
+    // object 700x900 24 vs 24, 1100^2 38 vs 35, 1900x1500 91 vs 68, blocks
+    // alone 1100^2 28 vs 35, 1500x1100 34 vs 42, 1900x1500 68 vs 65.
+    const bool flat2d = d->nz > 1 || (g.mat_E == MAT_UNIFORM && g.mat_H == MAT_UNIFORM) ||
+                        ncell < (d->n_objects > 0 ? 1200000 : 2500000);
+    const bool flat = !use_tma && d->precision == FDTD_FLOAT32 && p.n_shell == 0 && flat2d;
     p.flat = flat;
     if (!use_tma) {
         t.V = vec && !flat ? vmax : 1;
@@ -665,6 +699,16 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
         // active, its cells go to the shell (config 5 float32: z 32..172
         // would take three 64-cell tiles, the last 12 cells active; float32c:
         // 20..172, the last 24 of 64 active, 0.834 vs 0.804 ms per step)
+        // Where at most half of a 16-thread tile follows whole ones, it goes to
+        // the shell instead of up to half of a 32-thread tile idling: 223x224x64
+        // float64 476 -> 394 us per step, 202x203x78 418 -> 403; 126x127x100
+        // float32c 93 -> 83, 111x112x128 84 -> 82; 223x224x100 float32 186 ->
+        // 154, 197x198x128 161 -> 151.
+        const int zt = (bnz + t.V - 1) / t.V;
+        if (t.TZ == 32 && zt % 32 > 16 && zt % 16 <= 8 && zt % 16 != 0) {
+            t.TZ = 16;
+            t.TY = kThreads / 16;
+        }
         const int zc = t.V * t.TZ, rem = bnz % zc;
         if (rem != 0 && 2 * rem < zc && bnz > zc) {
             bnz -= rem;
@@ -865,7 +909,7 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
     }
 
     // what the fused passes apply, in order: the objects, and per half step the
-    // sources, a soft source of several points as one group (kItemSoftGroup)
+    // sources, an E source of several soft points as one group (kItemSoftGroup)
     struct Group {
         int item;
         std::vector<long long> cells;  // empty: the box is full
@@ -882,7 +926,7 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
         for (int q = first; q < last; q = e) {
             e = q + 1;
             while (e < last && items[e].source == items[q].source) ++e;
-            bool one = e - q > 1;
+            bool one = side == 0 && e - q > 1;
             for (int r = q; r < e; ++r)
                 one = one && items[r].kind == FDTD_ITEM_SOFT && items[r].comp == items[q].comp &&
                       items[r].column == items[q].column;
@@ -938,7 +982,7 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
         const int boxes[6][6] = {{0, 0, 0, lo[0], n[1], n[2]},         {hi[0], 0, 0, n[0], n[1], n[2]},
                                  {lo[0], 0, 0, hi[0], lo[1], n[2]},     {lo[0], hi[1], 0, hi[0], n[1], n[2]},
                                  {lo[0], lo[1], 0, hi[0], hi[1], lo[2]}, {lo[0], lo[1], hi[2], hi[0], hi[1], n[2]}};
-        const int sv = d->precision == FDTD_FLOAT64 ? shell_v<double>() : shell_v<float>();
+        const int sv = p.shell_v;
         long blocks = 0;
         for (const auto &b : boxes) {
             if (b[3] <= b[0] || b[4] <= b[1] || b[5] <= b[2]) continue;
@@ -1382,10 +1426,10 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
         p.kf.ez = ibox[5];
     }
     p.flat_general = flat && !flat_layers(p.kf, 2 * esize);
-    // the flat transposed half steps: float32 grids with every layer in the
-    // pass (the staged plans, split layers and partitions have their own)
+    // the flat transposed half steps: float32 grids whose layers are not in
+    // kernels of their own (staged plans have staged ones)
     p.kadj = p.k;
-    p.adj_flat = d->precision == FDTD_FLOAT32 && p.n_shell == 0 && p.pml_split == 0 &&
+    p.adj_flat = d->precision == FDTD_FLOAT32 && p.pml_split == 0 &&
                  flat_layers(p.kadj, 2 * esize);
     if (p.adj_flat) {
         const long chunks = ((long)d->ny * d->nz + kFlatBlock - 1) / kFlatBlock;
@@ -1477,7 +1521,8 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
         // Against one launch per half step, flat tiles, us per step: 64^3
         // 25.9 -> 14.4, 2D 1500x1100 43 -> 31, 128^3 55.6 -> 53.3, 131x150x97
         // 55.7 -> 54.3, but 192x192x96 112 -> 135; float64 register tiles
-        // 64^3 1.25x, 192x192x96 1.07x
+        // 64^3 70 -> 58, 128^3 309 -> 304 (larger float64 grids with layers
+        // are partitioned)
         const long auto_cells = d->precision == FDTD_FLOAT64 ? (8L << 20) : 3000000L;
         p.persistent = p.persist_ok && (d->persistent == 2 || (d->persistent == 0 && ncell < auto_cells));
         p.persist_blocks[0] = p.persist_blocks[1] = 0;

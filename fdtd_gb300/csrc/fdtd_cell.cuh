@@ -215,7 +215,9 @@ __device__ __forceinline__ SoftSpan soft_span(const ItemK &s, int ny, int nz, in
 }
 
 // Sources of one cell (fdtd/sources.py:93-109, 278-297, 476-486), in order.
-template <class P>
+// GROUPS: some may be soft-source groups (E half; the H half's lists have none,
+// whose registers would make the staged float32c pass spill).
+template <class P, bool GROUPS>
 __device__ __forceinline__ void apply_sources(const GridK &g, const int *idx, const double *__restrict__ wave, int i,
                                               int j, int k, typename P::T &fx, typename P::T &fy, typename P::T &fz,
                                               typename P::T &lx, typename P::T &ly, typename P::T &lz, int sb0,
@@ -225,23 +227,24 @@ __device__ __forceinline__ void apply_sources(const GridK &g, const int *idx, co
         const ItemK &s = g.items[idx[it]];
         if (!in_box(s, i, j, k)) continue;
         const T wv = (T)wave[s.column];
-        if (s.kind == kItemSoftGroup) {
-            const SoftSpan q = soft_span(s, g.ny, g.nz, i, j, k);
+        if (s.kind == FDTD_ITEM_SOFT || (GROUPS && s.kind == kItemSoftGroup)) {
+            // one loop for a point and for a group: two copies of the adds
+            // take registers that the staged passes do not have
+            const double *wt = &s.weight;
+            SoftSpan q{0, 1};
+            if (GROUPS && s.kind == kItemSoftGroup) {
+                q = soft_span(s, g.ny, g.nz, i, j, k);
+                wt = (const double *)s.coef[1];
+            }
+#pragma unroll 1
             for (int a = q.a; a < q.b; ++a) {
-                const T w = (T)((const double *)s.coef[1])[a];
+                const T w = (T)wt[a];
                 if (s.comp == 0) P::add_prod(fx, lx, w, wv);
                 else if (s.comp == 1) P::add_prod(fy, ly, w, wv);
                 else P::add_prod(fz, lz, w, wv);
             }
-            continue;
-        }
-        const T w = (T)s.weight;
-        if (s.kind == FDTD_ITEM_SOFT) {
-            if (s.comp == 0) P::add_prod(fx, lx, w, wv);
-            else if (s.comp == 1) P::add_prod(fy, ly, w, wv);
-            else P::add_prod(fz, lz, w, wv);
         } else {
-            const T val = P::mul(w, wv);
+            const T val = P::mul((T)s.weight, wv);
             if (s.comp == 0) P::set(fx, lx, val);
             else if (s.comp == 1) P::set(fy, ly, val);
             else P::set(fz, lz, val);
@@ -451,7 +454,7 @@ __device__ __forceinline__ void thread_E(const GridK &g, const double *__restric
 #pragma unroll
     for (int v = 0; v < V; ++v) {
         if (sb0 < sb1)
-            apply_sources<P>(g, g.srcE_idx, wave, i, j, k0 + v, e[3 * v], e[3 * v + 1], e[3 * v + 2], el[3 * v],
+            apply_sources<P, true>(g, g.srcE_idx, wave, i, j, k0 + v, e[3 * v], e[3 * v + 1], e[3 * v + 2], el[3 * v],
                              el[3 * v + 1], el[3 * v + 2], sb0, sb1);
         P::finish(e[3 * v], el[3 * v]);
         P::finish(e[3 * v + 1], el[3 * v + 1]);
@@ -490,7 +493,7 @@ __device__ __forceinline__ void thread_H(const GridK &g, const double *__restric
 #pragma unroll
     for (int v = 0; v < V; ++v) {
         if (sb0 < sb1)
-            apply_sources<P>(g, g.srcH_idx, wave, i, j, k0 + v, h[3 * v], h[3 * v + 1], h[3 * v + 2], hl[3 * v],
+            apply_sources<P, false>(g, g.srcH_idx, wave, i, j, k0 + v, h[3 * v], h[3 * v + 1], h[3 * v + 2], hl[3 * v],
                              hl[3 * v + 1], hl[3 * v + 2], sb0, sb1);
         P::finish(h[3 * v], hl[3 * v]);
         P::finish(h[3 * v + 1], hl[3 * v + 1]);

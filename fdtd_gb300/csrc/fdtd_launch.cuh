@@ -96,6 +96,12 @@ static void launch_flat(Plan &p, bool is_E, const double *wave, cudaStream_t st)
     else launch_flat_mat<P, MAT_FULL>(p, is_E, wave, st);
 }
 
+template <class P, int SV>
+static void launch_shell(Plan &p, bool is_E, const double *wave, unsigned blocks, cudaStream_t st) {
+    if (is_E) k_shell_E<P, SV><<<blocks, kThreads, 0, st>>>(p.kshell, p.shellk, wave);
+    else k_shell_H<P, SV><<<blocks, kThreads, 0, st>>>(p.kshell, p.shellk, wave);
+}
+
 // Staged-kernel tile shapes (threads along z x rows): 32x8, 32x4, 16x16.
 // The fused pass of a half step: one launch over the tile box and, for a
 // partitioned plan, one launch over the shell boxes, on the plan's second
@@ -122,9 +128,10 @@ static void launch_fused(Plan &p, bool is_E, const double *wave, cudaStream_t st
     if (p.n_shell) {
         const unsigned blocks = p.shellk.first[p.shellk.nbox];
         cudaStream_t ss = p.shell_overlap ? p.shell_stream : st;
-        constexpr int SV = shell_v<typename P::T>();
-        if (is_E) k_shell_E<P, SV><<<blocks, kThreads, 0, ss>>>(p.kshell, p.shellk, wave);
-        else k_shell_H<P, SV><<<blocks, kThreads, 0, ss>>>(p.kshell, p.shellk, wave);
+        if constexpr (sizeof(typename P::T) == 4) {
+            if (p.shell_v == 2) launch_shell<P, 2>(p, is_E, wave, blocks, ss);
+        }
+        if (p.shell_v == 1) launch_shell<P, 1>(p, is_E, wave, blocks, ss);
         if (p.shell_overlap) {
             cudaEventRecord(p.shell_join, ss);
             cudaStreamWaitEvent(st, p.shell_join, 0);
@@ -349,10 +356,15 @@ static int run_persistent(Plan &p, const fdtd_run_args *a, const fdtd_capture_ar
     pa.limit = 1u << 23;
     const void *fn = nullptr;
     dim3 block = p.block;
-    if constexpr (std::is_same<P, PF32>::value) {
-        fn = pa.n_curl ? persist_flat<P, true>(p.kf.mat_E, p.kf.mat_H)
-                       : persist_flat<P, false>(p.kf.mat_E, p.kf.mat_H);
+    if (p.flat) {
+        if constexpr (std::is_same<P, PF32>::value) {
+            fn = pa.n_curl ? persist_flat<P, true>(p.kf.mat_E, p.kf.mat_H)
+                           : persist_flat<P, false>(p.kf.mat_E, p.kf.mat_H);
+        }
         block = dim3(kFlatBlock);
+    } else if constexpr (std::is_same<P, PF32>::value) {  // 2D: one cell per thread
+        fn = p.kf.mat_H == MAT_UNIFORM ? (const void *)k_run_persistent<P, 1, MAT_FULL, MAT_UNIFORM>
+                                       : (const void *)k_run_persistent<P, 1, MAT_FULL, MAT_FULL>;
     } else if (p.kf.mat_H == MAT_UNIFORM) {
         fn = p.V > 1 ? (const void *)k_run_persistent<P, P::V, MAT_FULL, MAT_UNIFORM>
                      : (const void *)k_run_persistent<P, 1, MAT_FULL, MAT_UNIFORM>;
@@ -375,7 +387,7 @@ static int run_persistent(Plan &p, const fdtd_run_args *a, const fdtd_capture_ar
     pa.gz = (int)p.grid.x;
     pa.gy = (int)p.grid.y;
     pa.gx = (int)p.grid.z;
-    if (std::is_same<P, PF32>::value) {
+    if (p.flat) {
         // one tile per resident block where that keeps most of them busy, else the launch's tiles
         const long chunks = p.kf.flat_chunks;
         const long parts = std::min((long)p.kf.nx, resident / chunks);

@@ -181,12 +181,19 @@ __device__ __forceinline__ void persist_half(const GridK &g, const PersistArgs &
     }
 }
 
-// Flat tiles: three blocks of 80 registers (with four of 64 the two inlined
-// tiles spill 500 bytes).
+// Blocks per SM.  Flat tiles: three of 80 registers (with four of 64 the two
+// inlined tiles spill 500 bytes).  Register tiles: two; with one cell per
+// thread four (three in float64), which the compiler does not keep to by
+// itself (2D 520x454 float32c 16.6 us per step at 61 registers, 17.7 at 79).
+template <class P, int V>
+struct PersistTune {
+    static constexpr int blocks = V == 0 ? 3 : (V > 1 ? 2 : (sizeof(typename P::T) == 8 ? 3 : 4));
+};
+
 // CAP: steps that keep the curls of object boxes, apart from the plain run,
 // whose tiles would lose the registers (128^3: 52.9 -> 56.2 us per step).
 template <class P, int V, int MAT_E, int MAT_H, bool CAP = false>
-__global__ void __launch_bounds__(kThreads, V == 0 ? 3 : (V == 1 ? 1 : 2))
+__global__ void __launch_bounds__(kThreads, PersistTune<P, V>::blocks)
     k_run_persistent(const __grid_constant__ GridK g, const __grid_constant__ PersistArgs a) {
     using T = typename P::T;
     const int ntiles = a.gz * a.gy * a.gx;

@@ -91,6 +91,9 @@ struct Plan {
     // interior box; the n_shell boxes around it run one thread per cell with
     // every slab (kshell: the plan's GridK with per-block lists)
     int n_shell;
+    // cells per shell thread along z: two floats (even rows) or one value, which
+    // keeps the registers low enough for four blocks of 256 threads per SM
+    int shell_v;
     GridK kshell;
     ShellK shellk;
     // shell_overlap: the shell launch runs on a second stream beside the
