@@ -76,7 +76,7 @@ def parse():
     p.add_argument("--n", type=int, default=768, help="grid edge (config 3 is 768)")
     p.add_argument("--pml", type=int, default=-1, help="PML cells on y and z (default 20 scaled by n/768; 0 = none)")
     p.add_argument("--x-chunk", type=int, default=0, help="planes per CTA along x (0 = plan default)")
-    p.add_argument("--variant", type=int, default=0, help="0 auto, 1 register streaming, 2 TMA-staged")
+    p.add_argument("--variant", type=int, default=0, help="0 auto, 1 flat or register streaming, 2 TMA-staged")
     p.add_argument("--tile-rows", type=int, default=0)
     p.add_argument("--stages", type=int, default=0)
     p.add_argument("--pml-mode", type=int, default=0,

@@ -1509,7 +1509,7 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
         }
     }
 
-    // persistent time loop (fdtd_persistent.cuh): small register-streaming
+    // persistent time loop (fdtd_persistent.cuh): small flat or register-streaming
     // plans with nothing between the half steps but gathers and DFT sums
     if (d->persistent < 0 || d->persistent > 2) return FDTD_ERR_ARGUMENT;
     {
@@ -1519,7 +1519,7 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
                        p.n_current == 0 && (int)p.dft.size() <= kPersistMaxDft;
         // automatic: float32 and float32c below 3M cells, float64 below 8M.
         // Against one launch per half step, flat tiles, us per step: 64^3
-        // 25.9 -> 14.4, 2D 1500x1100 43 -> 31, 128^3 55.6 -> 53.3, 131x150x97
+        // 25.9 -> 12.5, 2D 1500x1100 43 -> 32, 128^3 55.6 -> 48.3, 131x150x97
         // 55.7 -> 54.3, but 192x192x96 112 -> 135; float64 register tiles
         // 64^3 70 -> 58, 128^3 309 -> 304 (larger float64 grids with layers
         // are partitioned)

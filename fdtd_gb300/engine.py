@@ -232,7 +232,7 @@ class Engine:
     def __init__(self, grid, x_chunk=0):
         self.grid = grid
         self.x_chunk = x_chunk
-        # fused-pass kernel choice: variant 0 auto / 1 register streaming / 2 TMA-staged
+        # fused-pass kernel choice: variant 0 auto / 1 flat or register streaming / 2 TMA-staged
         # materials: 0 compact copies for the staged passes where possible, 1 full arrays only
         # step_fusion: 0 auto / 1 two passes per step / 2 one pass per step (where allowed)
         # persistent: 0 auto / 1 one launch per half step / 2 one persistent launch per run() (where allowed)
@@ -347,8 +347,8 @@ class Engine:
 
     def set_tuning(self, variant=None, tile_rows=None, stages=None, x_chunk=None, pml_mode=None, materials=None,
                    step_fusion=None, persistent=None):
-        """Choose the fused-pass kernels (0 auto, 1 register streaming, 2 TMA-staged),
-        the TMA tile rows (4 or 8 with 32-thread-wide tiles, 16 with 16-wide) and
+        """Choose the fused-pass kernels (0 auto, 1 flat or register streaming,
+        2 TMA-staged), the TMA tile rows (4 or 8 with 32-thread-wide tiles, 16 with 16-wide) and
         ring stages, where the PML slabs run
         (0 auto, 1 inside the fused pass, 2 kernels of their own; 3 only the
         leading x/y slabs split off; 4 interior/shell partition: the fused
@@ -360,9 +360,10 @@ class Engine:
         currently never, the two-pass plans measured faster; 1 never; 2
         where the grid allows it, else RuntimeError); 0 keeps the automatic
         choice.  The one-pass step uses tile_rows 4 or 8, stages >= 3 and
-        x_chunk when given.  persistent: 0 auto (float32 grids below 3M
-        cells, float64 below 8M, whose plan allows it), 1 one launch per half step, 2 where allowed: every
-        full step of a run() in one cooperative launch."""
+        x_chunk when given.  persistent: 0 auto (float32 and
+        float32c grids below 3M cells, float64 below 8M, whose plan allows
+        it), 1 one launch per half step, 2 where allowed: every full step of a
+        run() in one cooperative launch."""
         for k, v in (("variant", variant), ("tile_rows", tile_rows), ("stages", stages), ("pml_mode", pml_mode),
                      ("materials", materials), ("step_fusion", step_fusion), ("persistent", persistent)):
             if v is not None:
@@ -382,7 +383,7 @@ class Engine:
         # their own, 2 interior/shell partition (the interior's tiling reported)
         info["pml_split"] = info["variant"] // 10
         info["variant"] %= 10
-        # 5: the persistent loop over register-streaming tiles
+        # 5: the persistent loop over flat or register-streaming tiles
         info["persistent"] = int(info["variant"] == 5)
         if info["persistent"]:
             info["variant"] = 1

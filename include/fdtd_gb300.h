@@ -132,7 +132,7 @@ typedef struct {
     int32_t precision;    /* fdtd_precision */
     int32_t nx, ny, nz;
     int32_t x_chunk;      /* planes per CTA along x; 0 = automatic */
-    int32_t variant;      /* fused-pass kernels: 0 automatic, 1 register streaming,
+    int32_t variant;      /* fused-pass kernels: 0 automatic, 1 flat or register streaming,
                              2 TMA-staged (needs nz a multiple of 4 floats / 2 doubles) */
     int32_t tile_rows;    /* TMA-staged: rows per CTA, 4 or 8 (tiles 32 threads wide along z)
                              or 16 (16 threads wide); 0 = automatic */
@@ -207,12 +207,12 @@ typedef struct {
      * buffer is allocated), whether the plan uses it, and why not. */
     int32_t step_fusion;
     /* Persistent time loop (ABI 5): on small grids whose plan runs the
-     * register-streaming passes with nothing between them but detector
+     * flat or register-streaming passes with nothing between them but detector
      * gathers and DFT sums, fdtd_run runs all full steps of a call in one
      * cooperative launch whose blocks meet at a grid-wide barrier between
      * half steps (bounded waits: bit 2 of the status word on expiry).  0
-     * automatic (float32 grids below 3M cells, float64 below 8M), 1 off, 2 on
-     * where the plan allows it. */
+     * automatic (float32 and float32c grids below 3M cells, float64 below 8M),
+     * 1 off, 2 on where the plan allows it. */
     int32_t persistent;
     void *E_alt;
     void *H_alt;
@@ -380,11 +380,11 @@ int fdtd_plan_step_fusion(const fdtd_plan *plan, int32_t *allowed, int32_t *acti
 
 /* Launch tiling chosen by the plan: out[0..7] = cells per thread along z,
  * threads along z, rows along y, planes along x per CTA, CTAs, kernels per
- * full step, variant (1 register streaming, 2 TMA-staged; plus 10 when the
+ * full step, variant (1 flat or register streaming, 2 TMA-staged; plus 10 when the
  * PML slabs run in kernels of their own, plus 20 for an interior/shell
  * partition, whose interior tiling is then reported; 4 one pass per full
  * step, whose tiling is then reported; 5 the persistent loop of
- * register-streaming tiles, one launch per fdtd_run call), ring stages. */
+ * flat or register-streaming tiles, one launch per fdtd_run call), ring stages. */
 int fdtd_plan_tiling(const fdtd_plan *plan, int64_t *out8);
 
 const char *fdtd_status_string(int32_t status);
