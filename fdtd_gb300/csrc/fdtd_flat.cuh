@@ -11,8 +11,8 @@
 // / thread_H, and so are the bits.
 //
 // Bound by latency and instruction issue, not by bytes: at 128^3 with 12-cell
-// layers (everything in L2) a half step issues 145 warp instructions per 32
-// cells, 37 % of the issue slots.  Four blocks of 64 registers per SM: five
+// layers (everything in L2) a half step issues 207 (E) and 167 (H) warp
+// instructions per 32 cells, 47 and 36 % of the issue slots.  Four blocks of 64 registers per SM: five
 // (48 registers) and three (80, two planes in flight in every loop) measured
 // slower, 56 and 59 against 43 us per step.  Against the register-streaming
 // tiles (four cells per thread, whose warps all hold a few cells of each z
