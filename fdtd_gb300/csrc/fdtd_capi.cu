@@ -9,6 +9,7 @@
 
 #include "fdtd_kernels.cuh"
 #include "fdtd_persistent.cuh"
+#include "fdtd_order.hpp"
 #include "fdtd_plan.hpp"
 
 struct fdtd_plan {
@@ -53,25 +54,16 @@ static int tile_width(int zt) {
 static bool flat_layers(GridK &g, size_t pair) {
     bool ok = g.nslab_fused == g.nslab;
     memset(g.lay, 0, sizeof(g.lay));
-    int axes[3], n = 0;
+    int axes[kMaxSlabs];
     for (int s = 0; s < g.nslab; ++s) {
         const SlabK &S = g.slab[s];
         ok = ok && g.lay[S.axis][S.high].th == 0 && ((uintptr_t)S.psiE | (uintptr_t)S.psiH) % pair == 0;
         g.lay[S.axis][S.high] = S;
-        int at = 0;
-        while (at < n && axes[at] != S.axis) ++at;
-        if (at == n) axes[n++] = S.axis;
-        else ok = ok && at == n - 1;
+        axes[s] = S.axis;
     }
-    for (int a = 0; a < 3; ++a) {
+    for (int a = 0; a < 3; ++a)
         ok = ok && (g.lay[a][0].th == 0 || g.lay[a][1].th == 0 || g.lay[a][0].th <= g.lay[a][1].start);
-        int at = 0;
-        while (at < n && axes[at] != a) ++at;
-        if (at == n) axes[n++] = a;
-    }
-    bool sorted = true;  // the plain order wherever it is as good as the registered one
-    for (int r = 0; r < 3; ++r) sorted = sorted && axes[r] == r;
-    g.lay_order = sorted ? 0x210 : (axes[0] | axes[1] << 4 | axes[2] << 8);
+    ok = layer_order(g.nslab, axes, g.lay_order) && ok;
     return ok;
 }
 
