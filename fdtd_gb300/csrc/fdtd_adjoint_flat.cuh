@@ -369,13 +369,13 @@ __global__ void __launch_bounds__(kFlatBlock, 4) k_adj_flat(const __grid_constan
                     v.f0 -= d1;
                 }
             };
-            if (g.lay_order == 0x210) {
+            if (g.lay_order == kOrderXYZ) {
                 layer(0);
                 layer(1);
                 layer(2);
             } else {
 #pragma unroll 1
-                for (int o = g.lay_order, r = 0; r < 3; ++r, o >>= 4) layer(o & 15);
+                for (int o = flat_order(g, i, j, k), r = 0; r < 3; ++r, o >>= 4) layer(o & 15);
             }
             pf[0] = v.f0;
             pf[1] = v.f1;

@@ -9,7 +9,6 @@
 
 #include "fdtd_kernels.cuh"
 #include "fdtd_persistent.cuh"
-#include "fdtd_order.hpp"
 #include "fdtd_plan.hpp"
 
 struct fdtd_plan {
@@ -49,21 +48,21 @@ static int tile_width(int zt) {
 
 // The layers of a flat pass by axis and side (GridK::lay); false where they
 // need the general form: two on one side, layers of one axis that share cells,
-// layers of two axes interleaved in boundary order, one behind a periodic
-// boundary, or auxiliaries that are not aligned to a pair.
+// one behind a periodic boundary, or auxiliaries that are not aligned to a pair.
 static bool flat_layers(GridK &g, size_t pair) {
     bool ok = g.nslab_fused == g.nslab;
     memset(g.lay, 0, sizeof(g.lay));
-    int axes[kMaxSlabs];
+    int axes[kMaxSlabs], high[kMaxSlabs];
     for (int s = 0; s < g.nslab; ++s) {
         const SlabK &S = g.slab[s];
         ok = ok && g.lay[S.axis][S.high].th == 0 && ((uintptr_t)S.psiE | (uintptr_t)S.psiH) % pair == 0;
         g.lay[S.axis][S.high] = S;
         axes[s] = S.axis;
+        high[s] = S.high;
     }
     for (int a = 0; a < 3; ++a)
         ok = ok && (g.lay[a][0].th == 0 || g.lay[a][1].th == 0 || g.lay[a][0].th <= g.lay[a][1].start);
-    ok = layer_order(g.nslab, axes, g.lay_order) && ok;
+    if (ok) g.lay_order = layer_order(g.nslab, axes, high, g.lay_rank);
     return ok;
 }
 

@@ -11,6 +11,7 @@
 #include <stdint.h>
 
 #include "../../include/fdtd_gb300.h"
+#include "fdtd_order.hpp"
 
 namespace fdtd {
 
@@ -89,7 +90,8 @@ struct GridK {
     int ox, oy, oz, ex, ey, ez;
     unsigned flat_chunks;            // flat half steps: blocks per plane of the box
     SlabK lay[3][2];                 // and the layers in the pass by axis and side (th 0: none),
-    int lay_order;                   // their axes in boundary order, four bits each from the lowest
+    int lay_order;                   // their axes in boundary order (fdtd_order.hpp),
+    LayerRank lay_rank;              // by side where they interleave
     FlatSources src_E, src_H;
     int stages;                      // shared-memory ring depth of the staged (TMA) kernels
     int *status;                     // device error word (bit 0: a pipeline wait timed out)

@@ -314,6 +314,12 @@ __device__ __forceinline__ void flat_source(const ItemK &s, int ny, int nz, cons
     }
 }
 
+// Order of a cell's layers.
+__device__ __forceinline__ int flat_order(const GridK &g, int i, int j, int k) {
+    if (g.lay_order != kOrderBySide) return g.lay_order;
+    return cell_order(g.lay_rank, i >= g.lay[0][0].th, j >= g.lay[1][0].th, k >= g.lay[2][0].th);
+}
+
 // What a thread knows of its column of a tile before it marches.  A block of
 // the persistent loop that keeps its tile works it out once per launch.
 template <class T>
@@ -534,7 +540,7 @@ __device__ __forceinline__ void flat_march(const GridK &g, const double *__restr
             if (hx) flat_psi<P>(X, qx, xz, xy);
             flat_psi<P>(Y, qy, yx, yz);
             flat_psi<P>(W, qw, zy, zx);
-            if (g.lay_order == 0x210) {
+            if (g.lay_order == kOrderXYZ) {
                 if (hx) pml_correct<P, IS_E>(v.f1, v.l1, v.m1, -qx.p0);
                 if (hx) pml_correct<P, IS_E>(v.f2, v.l2, v.m2, qx.p1);
                 if (hy) pml_correct<P, IS_E>(v.f2, v.l2, v.m2, -qy.p0);
@@ -543,7 +549,7 @@ __device__ __forceinline__ void flat_march(const GridK &g, const double *__restr
                 if (hw) pml_correct<P, IS_E>(v.f1, v.l1, v.m1, qw.p1);
             } else {
 #pragma unroll 1
-                for (int o = g.lay_order, r = 0; r < 3; ++r, o >>= 4) {
+                for (int o = flat_order(g, i, j, k), r = 0; r < 3; ++r, o >>= 4) {
                     if ((o & 15) == 0 && hx) {
                         pml_correct<P, IS_E>(v.f1, v.l1, v.m1, -qx.p0);
                         pml_correct<P, IS_E>(v.f2, v.l2, v.m2, qx.p1);

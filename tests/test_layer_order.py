@@ -18,11 +18,14 @@ HARNESS = r"""
 int main() {
     int n;
     while (scanf("%d", &n) == 1) {
-        int axis[6] = {0}, high[6] = {0}, order = 0;
+        int axis[6] = {0}, high[6] = {0};
         for (int s = 0; s < n; ++s)
             if (scanf("%d %d", &axis[s], &high[s]) != 2) return 1;
-        const bool one = fdtd::layer_order(n, axis, order);
-        printf("%d %d\n", (int)one, order);
+        fdtd::LayerRank rank;
+        const int order = fdtd::layer_order(n, axis, high, rank);
+        printf("%d %d", order != fdtd::kOrderBySide, order);
+        for (int c = 0; c < 8; ++c) printf(" %d", fdtd::cell_order(rank, c & 1, c & 2, c & 4));
+        printf("\n");
     }
 }
 """
@@ -62,6 +65,19 @@ def test_one_order_is_a_registration_order(orders):
         assert sorted(got) == [0, 1, 2]
         for s, t in itertools.combinations(reg, 2):
             assert s[0] == t[0] or got.index(s[0]) < got.index(t[0]), (reg, order)
+
+
+def test_order_of_a_cell_by_its_sides(orders):
+    """Layers of two axes that interleave: a cell's own layers in registration
+    order, whichever side of each axis it is on."""
+    sides = list(itertools.product(range(2), repeat=3))
+    assert any(not one for _, (one, *_) in orders)
+    for reg, (_, _, *cells) in orders:
+        for z, y, x in sides:
+            got = axes_of(cells[x + 2 * y + 4 * z])
+            assert sorted(got) == [0, 1, 2]
+            mine = [a for a, h in reg if h == (x, y, z)[a]]
+            assert [a for a in got if a in mine] == mine, (reg, got)
 
 
 def test_plain_order_wherever_the_layers_allow_it(orders):

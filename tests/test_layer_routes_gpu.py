@@ -1,0 +1,87 @@
+"""Absorbing layers registered in other orders than axis by axis: the plan that
+small float32 grids get, and the bits of the plan that corrects every layer in
+a kernel of its own, in registration order."""
+
+import numpy as np
+import pytest
+import torch
+
+from helpers import rel_l2
+from oracle import fdtd_oracle as fo
+from test_adjoint_flat_gpu import _gradient
+
+pytestmark = pytest.mark.gpu
+
+# (axis, high, thickness)
+INTERLEAVED = {
+    "lows_then_highs": [(0, 0, 4), (1, 0, 5), (2, 0, 3), (0, 1, 3), (1, 1, 4), (2, 1, 6)],
+    "highs_then_lows": [(2, 1, 6), (1, 1, 4), (0, 1, 3), (0, 0, 4), (2, 0, 3), (1, 0, 5)],
+    "z_split_by_y": [(2, 0, 3), (1, 0, 5), (1, 1, 4), (2, 1, 6)],
+    "x_split_by_z": [(0, 1, 3), (2, 1, 6), (0, 0, 4)],
+}
+
+
+def _layers(mod, g, spec):
+    for axis, high, t in spec:
+        if g.shape[axis] == 1:
+            continue
+        at = [slice(None)] * 3
+        at[axis] = slice(-t, None) if high else slice(0, t)
+        g[tuple(at)] = mod.PML()
+
+
+def _scene(mod, shape, spec):
+    nx, ny, nz = shape
+    eps = np.ones(shape)
+    eps[nx // 4:nx // 2, :, nz // 3:] = 4.0
+    g = mod.Grid(shape, grid_spacing=155e-9, permittivity=eps)
+    _layers(mod, g, spec)
+    g[3:nx - 3, 2:ny // 2, :] = mod.Object(permittivity=3.0)
+    g[nx // 2, ny // 2, nz // 2] = mod.PointSource(period=11)
+    g[:, ny // 2, nz // 2] = mod.LineDetector(name="line")
+    rng = np.random.default_rng(3)
+    g.E = rng.standard_normal(shape + (3,)).astype(np.float32).astype(np.float64)
+    g.H = rng.standard_normal(shape + (3,)).astype(np.float32).astype(np.float64)
+    return g
+
+
+def _run(fd, shape, spec, steps=12, **tune):
+    g = _scene(fd, shape, spec)
+    g._ensure_engine().set_tuning(**tune)
+    g.run(steps, progress_bar=False)
+    g._engine.check_status()
+    return g
+
+
+@pytest.mark.parametrize("shape", [(13, 17, 15), (16, 20, 32), (21, 40, 1)])
+@pytest.mark.parametrize("order", sorted(INTERLEAVED))
+def test_interleaved_layers(fd, order, shape):
+    fd.set_backend("gb300.float32")
+    spec = INTERLEAVED[order]
+    g = _run(fd, shape, spec)
+    assert g._engine.tiling()["persistent"] == 1
+    o = _scene(fo, shape, spec)
+    o.run(12)
+    assert rel_l2(g.E, o.E) <= 1e-4 and rel_l2(g.H, o.H) <= 1e-4
+    for tune in (dict(pml_mode=2, variant=1), dict(persistent=1), dict(persistent=2, x_chunk=3)):
+        f = _run(fd, shape, spec, **tune)
+        assert f._engine.tiling()["persistent"] == (tune.get("persistent") == 2)
+        assert torch.equal(f.E, g.E) and torch.equal(f.H, g.H), tune
+
+
+@pytest.mark.parametrize("order", sorted(INTERLEAVED))
+def test_gradient_through_interleaved_layers(fd, order):
+    def build(mod):
+        g = mod.Grid((12, 17, 18), grid_spacing=155e-9)
+        _layers(mod, g, [(a, h, min(t, 4)) for a, h, t in INTERLEAVED[order]])
+        obj = mod.Object(permittivity=2.0)
+        g[3:6, 4:9, 5:9] = obj
+        g[4, 6, 9] = mod.PointSource(period=9)
+        g[:, 7, 9] = mod.LineDetector(name="line")
+        value = np.random.default_rng(5).uniform(0.3, 0.9, size=(3, 5, 4))
+        return g, obj, value, {("line", "E"): np.ones(3), ("line", "H"): np.full(3, 0.5)}, 5
+
+    flat = _gradient(fd, build, "float32", pml_mode=1, variant=1)
+    assert np.abs(flat).max() > 0
+    assert np.array_equal(flat, _gradient(fd, build, "float32", pml_mode=2, variant=1))
+    assert rel_l2(flat, _gradient(fd, build, "float64")) <= 1e-4
