@@ -46,9 +46,9 @@ static int tile_width(int zt) {
     return pad16 < pad32 ? 16 : 32;
 }
 
-// The layers of a flat pass by axis and side (GridK::lay); false where they
-// need the general form: two on one side, layers of one axis that share cells,
-// one behind a periodic boundary, or auxiliaries that are not aligned to a pair.
+// The layers of a flat pass by axis and side (GridK::lay); false where it does
+// not take them: two on one side, layers of one axis that share cells, one
+// behind a periodic boundary, or auxiliaries that are not aligned to a pair.
 static bool flat_layers(GridK &g, size_t pair) {
     bool ok = g.nslab_fused == g.nslab;
     memset(g.lay, 0, sizeof(g.lay));
@@ -676,10 +676,24 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
     // alone 1100^2 28 vs 35, 1500x1100 34 vs 42, 1900x1500 68 vs 65.
     const bool flat2d = d->nz > 1 || (g.mat_E == MAT_UNIFORM && g.mat_H == MAT_UNIFORM) ||
                         ncell < (d->n_objects > 0 ? 1200000 : 2500000);
-    const bool flat = !use_tma && d->precision == FDTD_FLOAT32 && p.n_shell == 0 && flat2d;
+    // Layers that the flat passes do not take (flat_layers) keep the register
+    // tiles, which stay in the persistent loop.  us per step, a general flat
+    // form (one launch per half step) vs register: layers of one axis that
+    // share cells 64^3 25.6 vs 16.9, 128^3 121 vs 82, 2D 1400^2 95 vs 72,
+    // 2D 2500^2 220 vs 190, 255x251x249 496 vs 474; z layers behind a periodic
+    // y 64^3 54 vs 51, 192x192x96 165 vs 160, 255x251x249 474 vs 374, but
+    // 100^3 69 vs 74 and 128x128x96 87 vs 96.
+    GridK inside = g;  // with the layers inside the pass
+    inside.nslab = ks;
+    inside.nslab_fused = std::min(g.nslab_fused, ks);
+    const bool flat = !use_tma && d->precision == FDTD_FLOAT32 && p.n_shell == 0 && flat2d &&
+                      flat_layers(inside, 2 * esize);
     p.flat = flat;
     if (!use_tma) {
-        t.V = vec && !flat ? vmax : 1;
+        // (the vector tiles load auxiliaries 16 bytes at a time)
+        bool psi16 = true;
+        for (int s = 0; s < ks; ++s) psi16 = psi16 && aligned16(g.slab[s].psiE) && aligned16(g.slab[s].psiH);
+        t.V = vec && psi16 && !flat ? vmax : 1;
         t.TZ = flat ? kFlatBlock : tile_width((bnz + t.V - 1) / t.V);
         t.TY = flat ? 1 : kThreads / t.TZ;
         g.stages = 0;
@@ -1416,7 +1430,7 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
         p.kf.ey = ibox[4];
         p.kf.ez = ibox[5];
     }
-    p.flat_general = flat && !flat_layers(p.kf, 2 * esize);
+    if (flat) flat_layers(p.kf, 2 * esize);
     // the flat transposed half steps: float32 grids whose layers are not in
     // kernels of their own (staged plans have staged ones)
     p.kadj = p.k;
@@ -1506,7 +1520,7 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
     {
         int coop = 0;
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-        p.persist_ok = coop && p.variant == 1 && !p.flat_general && p.n_shell == 0 && p.epi_E.empty() && p.epi_H.empty() && !p.has_feedback &&
+        p.persist_ok = coop && p.variant == 1 && p.n_shell == 0 && p.epi_E.empty() && p.epi_H.empty() && !p.has_feedback &&
                        p.n_current == 0 && (int)p.dft.size() <= kPersistMaxDft;
         // automatic: float32 and float32c below 3M cells, float64 below 8M.
         // Against one launch per half step, flat tiles, us per step: 64^3

@@ -581,77 +581,14 @@ __device__ __forceinline__ void flat_march(const GridK &g, const double *__restr
     }
 }
 
-template <class P, bool IS_E, int MAT>
-__device__ __forceinline__ void flat_tile(const GridK &g, const double *__restrict__ wave, unsigned chunk, int xa,
-                                          int xb) {
-    flat_march<P, IS_E, MAT>(g, wave, chunk, xa, xb, flat_column<P, IS_E>(g, chunk, xa, xb));
-}
-
-// The same with the per-cell body of the staged passes, which takes layers of
-// one axis that share cells, in any order and corrected later (a layer behind
-// a periodic boundary), and auxiliaries of any alignment.
-template <class P, bool IS_E>
-__device__ __forceinline__ void flat_tile_general(const GridK &g, const double *__restrict__ wave, unsigned chunk,
-                                                  int xa, int xb) {
-    using T = typename P::T;
-    const FlatPlace pl = flat_place(g, chunk);
-    if (!pl.in) return;
-    const int j = pl.j, k = pl.k, ny = g.ny, nz = g.nz;
-    const T *N = (const T *)(IS_E ? g.H : g.E);
-    T *F = (T *)(IS_E ? g.E : g.H);
-    T *Flo = (T *)(IS_E ? g.Elo : g.Hlo);
-    const T *M = (const T *)(IS_E ? g.ie : g.imu);
-    const T c = courant_of<T>(g);
-    const unsigned mask_yz = slab_mask_yz(g, j, k, 1);
-    const PsiSrc<T> nostage{nullptr, 0, 0, nullptr};
-    int sb0 = 0, sb1 = 0;
-    if (IS_E ? g.fuse_src_E : g.fuse_src_H) {
-        const int *off = IS_E ? g.srcE_off : g.srcH_off;
-        sb0 = off[chunk];
-        sb1 = off[chunk + 1];
-    }
-    for (int i = xa; i < xb; ++i) {
-        const long v = 3 * (((long)i * ny + j) * nz + k), d = IS_E ? -1 : 1;
-        T a[3], x[3] = {T(0), T(0), T(0)}, y[3] = {T(0), T(0), T(0)}, f[3], fl[3] = {T(0), T(0), T(0)}, m[3];
-        T kx = T(0), ky = T(0);
-        const bool xok = IS_E ? i > 0 : i < g.nx - 1, yok = IS_E ? j > 0 : j < ny - 1,
-                   zok = IS_E ? k > 0 : k < nz - 1;
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-            a[q] = N[v + q];
-            if (xok) x[q] = N[v + d * 3L * ny * nz + q];
-            if (yok) y[q] = N[v + d * 3L * nz + q];
-            f[q] = F[v + q];
-            if constexpr (P::COMP) fl[q] = Flo[v + q];
-            m[q] = M[v + q];
-        }
-        if (zok) {
-            kx = N[v + 3 * d];
-            ky = N[v + 3 * d + 1];
-        }
-        const unsigned slabs = mask_yz | slab_mask_x(g, i);
-        if constexpr (IS_E)
-            thread_E<P, 1>(g, wave, i, j, k, c, a, x, y, kx, ky, m, f, fl, g.obj_off[chunk], g.obj_off[chunk + 1], sb0,
-                           sb1, nostage, slabs);
-        else
-            thread_H<P, 1>(g, wave, i, j, k, c, a, x, y, kx, ky, m, f, fl, sb0, sb1, nostage, slabs);
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-            F[v + q] = f[q];
-            if constexpr (P::COMP) Flo[v + q] = fl[q];
-        }
-    }
-}
-
 // Block b of a half step: chunk b mod n of the plane, x chunk b / n.  MAT: how
-// the material is read, or -1 for the general form.
+// the material is read.
 template <class P, bool IS_E, int MAT>
 __global__ void __launch_bounds__(kFlatBlock, FlatTune<P>::blocks)
     k_flat(const __grid_constant__ GridK g, const double *__restrict__ wave) {
     const unsigned n = g.flat_chunks, xc = blockIdx.x / n, chunk = blockIdx.x - xc * n;
     const int xa = g.ox + (int)xc * g.XC, xb = min(g.ex, xa + g.XC);
-    if constexpr (MAT < 0) flat_tile_general<P, IS_E>(g, wave, chunk, xa, xb);
-    else flat_tile<P, IS_E, MAT>(g, wave, chunk, xa, xb);
+    flat_march<P, IS_E, MAT>(g, wave, chunk, xa, xb, flat_column<P, IS_E>(g, chunk, xa, xb));
 }
 
 }  // namespace fdtd

@@ -89,9 +89,8 @@ static void launch_flat_mat(Plan &p, bool is_E, const double *wave, cudaStream_t
 
 template <class P>
 static void launch_flat(Plan &p, bool is_E, const double *wave, cudaStream_t st) {
-    const int mat = p.flat_general ? -1 : (is_E ? p.kf.mat_E : p.kf.mat_H);
-    if (mat < 0) launch_flat_mat<P, -1>(p, is_E, wave, st);
-    else if (mat == MAT_UNIFORM) launch_flat_mat<P, MAT_UNIFORM>(p, is_E, wave, st);
+    const int mat = is_E ? p.kf.mat_E : p.kf.mat_H;
+    if (mat == MAT_UNIFORM) launch_flat_mat<P, MAT_UNIFORM>(p, is_E, wave, st);
     else if (mat == MAT_IDS) launch_flat_mat<P, MAT_IDS>(p, is_E, wave, st);
     else launch_flat_mat<P, MAT_FULL>(p, is_E, wave, st);
 }
@@ -362,9 +361,6 @@ static int run_persistent(Plan &p, const fdtd_run_args *a, const fdtd_capture_ar
                            : persist_flat<P, false>(p.kf.mat_E, p.kf.mat_H);
         }
         block = dim3(kFlatBlock);
-    } else if constexpr (std::is_same<P, PF32>::value) {  // 2D: one cell per thread
-        fn = p.kf.mat_H == MAT_UNIFORM ? (const void *)k_run_persistent<P, 1, MAT_FULL, MAT_UNIFORM>
-                                       : (const void *)k_run_persistent<P, 1, MAT_FULL, MAT_FULL>;
     } else if (p.kf.mat_H == MAT_UNIFORM) {
         fn = p.V > 1 ? (const void *)k_run_persistent<P, P::V, MAT_FULL, MAT_UNIFORM>
                      : (const void *)k_run_persistent<P, 1, MAT_FULL, MAT_UNIFORM>;

@@ -35,9 +35,7 @@ struct Plan {
     int V;             // cells per thread along z (flat: 1)
     dim3 grid, block;  // fused-pass launch shape
     int variant;       // 1 flat or register streaming, 2 TMA-staged
-    int flat;          // variant 1 runs the flat half steps: float32 but the interior of a partition
-    int flat_general;  // flat half steps in their general form: PML slabs of one axis share cells, or
-                       // auxiliaries not aligned to a pair
+    int flat;          // variant 1 runs the flat half steps
     size_t smem_bytes; // dynamic shared memory of the TMA-staged kernels
     CUtensorMap maps[MAP_COUNT];
     const void *index_E, *index_H;  // one-byte material indices (MAT_IDS)

@@ -85,3 +85,26 @@ def test_gradient_through_interleaved_layers(fd, order):
     assert np.abs(flat).max() > 0
     assert np.array_equal(flat, _gradient(fd, build, "float32", pml_mode=2, variant=1))
     assert rel_l2(flat, _gradient(fd, build, "float64")) <= 1e-4
+
+
+# layers that the flat passes do not take
+OTHERS = {
+    "share_x": [(0, 0, 9), (0, 1, 8), (1, 0, 3), (1, 1, 4)],
+    "share_all": [(0, 0, 9), (2, 0, 9), (1, 0, 12), (0, 1, 8), (1, 1, 9), (2, 1, 10)],
+}
+
+
+@pytest.mark.parametrize("shape", [(13, 17, 15), (16, 20, 16), (14, 40, 1)])
+@pytest.mark.parametrize("spec", sorted(OTHERS))
+def test_layers_of_one_axis_that_share_cells(fd, spec, shape):
+    fd.set_backend("gb300.float32")
+    spec = OTHERS[spec]
+    g = _run(fd, shape, spec)
+    assert g._engine.tiling()["persistent"] == 1
+    o = _scene(fo, shape, spec)
+    o.run(12)
+    assert rel_l2(g.E, o.E) <= 1e-4 and rel_l2(g.H, o.H) <= 1e-4
+    for tune in (dict(pml_mode=2, variant=1), dict(persistent=1), dict(persistent=2, x_chunk=3)):
+        f = _run(fd, shape, spec, **tune)
+        assert f._engine.tiling()["persistent"] == (tune.get("persistent") == 2)
+        assert torch.equal(f.E, g.E) and torch.equal(f.H, g.H), tune
