@@ -183,11 +183,14 @@ __device__ __forceinline__ void persist_half(const GridK &g, const PersistArgs &
 
 // Blocks per SM.  Flat tiles: three of 80 registers (with four of 64 the two
 // inlined tiles spill 500 bytes).  Register tiles: two; with one cell per
-// thread four (three in float64), which the compiler does not keep to by
-// itself (2D 520x454 float32c 16.6 us per step at 61 registers, 17.7 at 79).
+// thread five in float32, four in float32c and three in float64, which the
+// compiler does not keep to by itself (2D 520x454 float32c 16.6 us per step at
+// 61 registers, 17.7 at 79; float32 at 48 and 56 registers: 2D 1500^2 with an
+// object 56.2 and 61.4, 1700^2 63.1 and 65.3, 131x150x97 with layers that share
+// cells 74.5 and 80.4).
 template <class P, int V>
 struct PersistTune {
-    static constexpr int blocks = V == 0 ? 3 : (V > 1 ? 2 : (sizeof(typename P::T) == 8 ? 3 : 4));
+    static constexpr int blocks = V == 0 ? 3 : (V > 1 ? 2 : (sizeof(typename P::T) == 8 ? 3 : (P::COMP ? 4 : 5)));
 };
 
 // CAP: steps that keep the curls of object boxes, apart from the plain run,
