@@ -27,14 +27,7 @@
 
 namespace fdtd {
 
-// Blocks per SM the kernels are compiled for, and whether the short loop loads
-// two planes before it computes the first (only where that leaves these blocks
-// resident).
-template <class P>
-struct FlatTune {
-    static constexpr int blocks = sizeof(typename P::T) == 8 ? 3 : 4;
-    static constexpr bool pairs = sizeof(typename P::T) == 4 && !P::COMP;
-};
+constexpr int kFlatBlocks = 4;  // per SM
 
 // A pair of auxiliaries of a layer, or of values.
 template <class T>
@@ -52,26 +45,15 @@ struct FlatLayer {
     bool inc;
 };
 
-// The pair of a layer on one plane, updated with its two differences and stored.
+// The pair of a layer on one plane, updated with its two differences and
+// stored (without the drive: p b + 0 c).
 template <class P>
 __device__ __forceinline__ void flat_psi(const FlatLayer<typename P::T> &L, FlatPair<typename P::T> &p,
                                          typename P::T d0, typename P::T d1) {
     using T = typename P::T;
-    if constexpr (sizeof(T) == 4) {
-        // (without the drive: p b + 0 c)
-        p.p0 = P::psi(p.p0, L.b, L.inc ? d0 : T(0), L.c);
-        p.p1 = P::psi(p.p1, L.b, L.inc ? d1 : T(0), L.c);
-        if (L.q) *L.q = p;
-    } else if (L.q) {
-        if (L.inc) {
-            p.p0 = P::psi(p.p0, L.b, d0, L.c);
-            p.p1 = P::psi(p.p1, L.b, d1, L.c);
-        } else {
-            p.p0 = P::mul(p.p0, L.b);
-            p.p1 = P::mul(p.p1, L.b);
-        }
-        *L.q = p;
-    }
+    p.p0 = P::psi(p.p0, L.b, L.inc ? d0 : T(0), L.c);
+    p.p1 = P::psi(p.p1, L.b, L.inc ? d1 : T(0), L.c);
+    if (L.q) *L.q = p;
 }
 
 // Column of a block's thread in the plane of the tile box.
@@ -96,56 +78,48 @@ __device__ __forceinline__ FlatPlace flat_place(const GridK &g, unsigned chunk) 
     return p;
 }
 
+// One source on a cell of its box: x is the cell's value of the source's component.
+template <class P>
+__device__ __forceinline__ void flat_source(const ItemK &s, int ny, int nz, const double *__restrict__ wave, int i,
+                                            int j, int k, typename P::T &x) {
+    using T = typename P::T;
+    T none = T(0);
+    const T wv = (T)wave[s.column];
+    if (s.kind == kItemSoftGroup) {
+        const SoftSpan q = soft_span(s, ny, nz, i, j, k);
+        for (int a = q.a; a < q.b; ++a) P::add_prod(x, none, (T)((const double *)s.coef[1])[a], wv);
+    } else if (s.kind == FDTD_ITEM_SOFT) {
+        P::add_prod(x, none, (T)s.weight, wv);
+    } else {
+        P::set(x, none, P::mul((T)s.weight, wv));
+    }
+}
+
 // The n sources in idx on the thread's cell of planes [xa, xb), in order, after
-// the march has stored those planes (compensated pairs not yet normalised).
+// the march has stored those planes.
 template <class P>
 __device__ __forceinline__ void flat_sources(const GridK &g, const int *idx, int n, const double *__restrict__ wave,
-                                             int xa, int xb, int j, int k, long jk, typename P::T *F,
-                                             typename P::T *Flo) {
+                                             int xa, int xb, int j, int k, long jk, typename P::T *F) {
     using T = typename P::T;
     for (int i = xa; i < xb; ++i) {
-        T *f = F + 3 * ((long)i * g.ny * g.nz + jk), *fl = P::COMP ? Flo + (f - F) : nullptr;
-        T y[3] = {T(0), T(0), T(0)};
-        if constexpr (P::COMP) {
-            for (int c = 0; c < 3; ++c) y[c] = fl[c];
-        }
+        T *f = F + 3 * ((long)i * g.ny * g.nz + jk);
         for (int it = 0; it < n; ++it) {
             const ItemK &s = g.items[idx[it]];
             if (!in_box(s, i, j, k)) continue;
-            const int c = s.comp;
-            T x = f[c], l = c == 0 ? y[0] : (c == 1 ? y[1] : y[2]);
-            const T wv = (T)wave[s.column];
-            if (s.kind == kItemSoftGroup) {
-                const SoftSpan q = soft_span(s, g.ny, g.nz, i, j, k);
-                for (int a = q.a; a < q.b; ++a) P::add_prod(x, l, (T)((const double *)s.coef[1])[a], wv);
-            } else if (s.kind == FDTD_ITEM_SOFT) {
-                P::add_prod(x, l, (T)s.weight, wv);
-            } else {
-                P::set(x, l, P::mul((T)s.weight, wv));
-            }
-            f[c] = x;
-            if (c == 0) y[0] = l;
-            else if (c == 1) y[1] = l;
-            else y[2] = l;
-        }
-        if constexpr (P::COMP) {
-            for (int c = 0; c < 3; ++c) {
-                T x = f[c];
-                P::finish(x, y[c]);
-                f[c] = x;
-                fl[c] = y[c];
-            }
+            T x = f[s.comp];
+            flat_source<P>(s, g.ny, g.nz, wave, i, j, k, x);
+            f[s.comp] = x;
         }
     }
 }
 
 // Where a thread stands in its march: its cell of the present plane in the
-// neighbour field, the field, its compensation and the material (values or
-// index), and the neighbour field on the plane before.
+// neighbour field, the field and the material (values or index), and the
+// neighbour field on the plane before.
 template <class T>
 struct FlatMarch {
     const T *pn;
-    T *pf, *plo;
+    T *pf;
     const T *pm;
     const unsigned char *pid;
     T by, bz;
@@ -155,7 +129,7 @@ struct FlatMarch {
 // neighbours, the field, courant times the material.
 template <class T>
 struct FlatCell {
-    T ax, ay, az, yx, yz, zx, zy, f0, f1, f2, l0, l1, l2, m0, m1, m2;
+    T ax, ay, az, yx, yz, zx, zy, f0, f1, f2, m0, m1, m2;
     int id;
 };
 
@@ -174,12 +148,6 @@ __device__ __forceinline__ void flat_load(FlatCell<typename P::T> &v, const Flat
     v.f0 = f[0];
     v.f1 = f[1];
     v.f2 = f[2];
-    v.l0 = v.l1 = v.l2 = typename P::T(0);
-    if constexpr (P::COMP) {
-        v.l0 = s.plo[step];
-        v.l1 = s.plo[step + 1];
-        v.l2 = s.plo[step + 2];
-    }
     if constexpr (MAT == MAT_FULL) {
         v.m0 = s.pm[step];
         v.m1 = s.pm[step + 1];
@@ -213,14 +181,15 @@ __device__ __forceinline__ void flat_material(FlatCell<typename P::T> &v, const 
 template <class P, bool IS_E>
 __device__ __forceinline__ void flat_bulk(FlatCell<typename P::T> &v, typename P::T u0, typename P::T u1,
                                           typename P::T u2) {
+    typename P::T none = 0;
     if (IS_E) {
-        P::add_prod(v.f0, v.l0, v.m0, u0);
-        P::add_prod(v.f1, v.l1, v.m1, u1);
-        P::add_prod(v.f2, v.l2, v.m2, u2);
+        P::add_prod(v.f0, none, v.m0, u0);
+        P::add_prod(v.f1, none, v.m1, u1);
+        P::add_prod(v.f2, none, v.m2, u2);
     } else {
-        P::sub_prod(v.f0, v.l0, v.m0, u0);
-        P::sub_prod(v.f1, v.l1, v.m1, u1);
-        P::sub_prod(v.f2, v.l2, v.m2, u2);
+        P::sub_prod(v.f0, none, v.m0, u0);
+        P::sub_prod(v.f1, none, v.m1, u1);
+        P::sub_prod(v.f2, none, v.m2, u2);
     }
 }
 
@@ -237,34 +206,20 @@ __device__ __forceinline__ void flat_plain(FlatCell<typename P::T> &v, typename 
     flat_bulk<P, IS_E>(v, yz - zy, zx - xz, xy - yx);
 }
 
-// The cell stored, normalised unless sources follow.
-template <class P>
-__device__ __forceinline__ void flat_store(FlatCell<typename P::T> &v, const FlatMarch<typename P::T> &s, bool last,
-                                           long step) {
-    if (last) {
-        P::finish(v.f0, v.l0);
-        P::finish(v.f1, v.l1);
-        P::finish(v.f2, v.l2);
-    }
+template <class T>
+__device__ __forceinline__ void flat_store(const FlatCell<T> &v, const FlatMarch<T> &s, long step) {
     s.pf[step] = v.f0;
     s.pf[step + 1] = v.f1;
     s.pf[step + 2] = v.f2;
-    if constexpr (P::COMP) {
-        s.plo[step] = v.l0;
-        s.plo[step + 1] = v.l1;
-        s.plo[step + 2] = v.l2;
-    }
 }
 
 // The march moved on by `step` values past cell v.
-template <class P, int MAT>
-__device__ __forceinline__ void flat_next(FlatMarch<typename P::T> &s, const FlatCell<typename P::T> &v, long step,
-                                          long istep) {
+template <class T, int MAT>
+__device__ __forceinline__ void flat_next(FlatMarch<T> &s, const FlatCell<T> &v, long step, long istep) {
     s.by = v.ay;
     s.bz = v.az;
     s.pn += step;
     s.pf += step;
-    if constexpr (P::COMP) s.plo += step;
     if constexpr (MAT == MAT_FULL) s.pm += step;
     if constexpr (MAT == MAT_IDS) s.pid += istep;
 }
@@ -285,33 +240,6 @@ __device__ __forceinline__ FlatLayer<T> flat_layer_at(const SlabK (&lay)[2], int
     L.c = ((const T *)(IS_E ? (low ? A.cE : B.cE) : (low ? A.cH : B.cH)))[l];
     L.inc = IS_E ? l >= 1 : l <= (low ? A.th : B.th) - 2;
     return L;
-}
-
-// One source on a cell of its box.
-template <class P>
-__device__ __forceinline__ void flat_source(const ItemK &s, int ny, int nz, const double *__restrict__ wave, int i,
-                                            int j, int k, FlatCell<typename P::T> &v) {
-    using T = typename P::T;
-    T x = s.comp == 0 ? v.f0 : (s.comp == 1 ? v.f1 : v.f2), l = s.comp == 0 ? v.l0 : (s.comp == 1 ? v.l1 : v.l2);
-    const T wv = (T)wave[s.column];
-    if (s.kind == kItemSoftGroup) {
-        const SoftSpan q = soft_span(s, ny, nz, i, j, k);
-        for (int a = q.a; a < q.b; ++a) P::add_prod(x, l, (T)((const double *)s.coef[1])[a], wv);
-    } else if (s.kind == FDTD_ITEM_SOFT) {
-        P::add_prod(x, l, (T)s.weight, wv);
-    } else {
-        P::set(x, l, P::mul((T)s.weight, wv));
-    }
-    if (s.comp == 0) {
-        v.f0 = x;
-        v.l0 = l;
-    } else if (s.comp == 1) {
-        v.f1 = x;
-        v.l1 = l;
-    } else {
-        v.f2 = x;
-        v.l2 = l;
-    }
 }
 
 // Order of a cell's layers.
@@ -410,6 +338,7 @@ template <class P, bool IS_E, int MAT>
 __device__ __forceinline__ void flat_march(const GridK &g, const double *__restrict__ wave, unsigned chunk, int xa,
                                            int xb, const FlatColumn<typename P::T> &col) {
     using T = typename P::T;
+    static_assert(sizeof(T) == 4 && !P::COMP, "float32 only: see the head of this file");
     constexpr int dir = IS_E ? 1 : -1;
     if (!col.in) return;
     const int nx = g.nx, ny = g.ny, nz = g.nz;
@@ -432,7 +361,6 @@ __device__ __forceinline__ void flat_march(const GridK &g, const double *__restr
     FlatMarch<T> s;
     s.pn = (const T *)(IS_E ? g.H : g.E) + 3 * first;
     s.pf = (T *)(IS_E ? g.E : g.H) + 3 * first;
-    s.plo = P::COMP ? (T *)(IS_E ? g.Elo : g.Hlo) + 3 * first : nullptr;
     s.pm = MAT == MAT_FULL ? (const T *)(IS_E ? g.ie : g.imu) + 3 * first : nullptr;
     s.pid = MAT == MAT_IDS ? (IS_E ? g.mid_E : g.mid_H) + first : nullptr;
     T m[3] = {T(0), T(0), T(0)};
@@ -471,20 +399,18 @@ __device__ __forceinline__ void flat_march(const GridK &g, const double *__restr
             }
         }
         if (!special && tb == nullptr && xok) {
-            if constexpr (FlatTune<P>::pairs) {
 #pragma unroll 1
-                for (; (stop - i) * dir >= 2; i += 2 * dir) {
-                    FlatCell<T> v, w;
-                    flat_load<P, MAT>(v, s, 0, 0, oy, oz);
-                    flat_load<P, MAT>(w, s, step, istep, oy, oz);
-                    flat_material<P, MAT>(v, lut, nlut, courant, m);
-                    flat_plain<P, IS_E>(v, s.by, s.bz, nz == 1);
-                    flat_store<P>(v, s, listed == 0, 0);
-                    flat_material<P, MAT>(w, lut, nlut, courant, m);
-                    flat_plain<P, IS_E>(w, v.ay, v.az, nz == 1);
-                    flat_store<P>(w, s, listed == 0, step);
-                    flat_next<P, MAT>(s, w, 2 * step, 2 * istep);
-                }
+            for (; (stop - i) * dir >= 2; i += 2 * dir) {
+                FlatCell<T> v, w;
+                flat_load<P, MAT>(v, s, 0, 0, oy, oz);
+                flat_load<P, MAT>(w, s, step, istep, oy, oz);
+                flat_material<P, MAT>(v, lut, nlut, courant, m);
+                flat_plain<P, IS_E>(v, s.by, s.bz, nz == 1);
+                flat_store(v, s, 0);
+                flat_material<P, MAT>(w, lut, nlut, courant, m);
+                flat_plain<P, IS_E>(w, v.ay, v.az, nz == 1);
+                flat_store(w, s, step);
+                flat_next<T, MAT>(s, w, 2 * step, 2 * istep);
             }
 #pragma unroll 1
             for (; i != stop; i += dir) {
@@ -492,8 +418,8 @@ __device__ __forceinline__ void flat_march(const GridK &g, const double *__restr
                 flat_load<P, MAT>(v, s, 0, 0, oy, oz);
                 flat_material<P, MAT>(v, lut, nlut, courant, m);
                 flat_plain<P, IS_E>(v, s.by, s.bz, nz == 1);
-                flat_store<P>(v, s, listed == 0, 0);
-                flat_next<P, MAT>(s, v, step, istep);
+                flat_store(v, s, 0);
+                flat_next<T, MAT>(s, v, step, istep);
             }
             continue;
         }
@@ -520,19 +446,20 @@ __device__ __forceinline__ void flat_march(const GridK &g, const double *__restr
             const T zx = zok ? (IS_E ? v.ax - v.zx : v.zx - v.ax) : T(0);
             const T zy = zok ? (IS_E ? v.ay - v.zy : v.zy - v.ay) : T(0);
             const T u0 = yz - zy, u1 = zx - xz, u2 = xy - yx;
+            T none = T(0);
             flat_bulk<P, IS_E>(v, u0, u1, u2);
             if constexpr (IS_E) {
                 for (unsigned om = omask; om; om &= om - 1) {
                     const ItemK &o = g.items[g.obj_idx[ob0 + __ffs(om) - 1]];
                     if (i >= o.lo[0] && i < o.hi[0])
-                        apply_object_cell<P>(o, box_index(o, i, j, k), courant, u0, u1, u2, v.f0, v.f1, v.f2, v.l0,
-                                             v.l1, v.l2);
+                        apply_object_cell<P>(o, box_index(o, i, j, k), courant, u0, u1, u2, v.f0, v.f1, v.f2, none,
+                                             none, none);
                 }
                 for (int it = ob0 + 32; it < ob1; ++it) {
                     const ItemK &o = g.items[g.obj_idx[it]];
                     if (in_box(o, i, j, k))
-                        apply_object_cell<P>(o, box_index(o, i, j, k), courant, u0, u1, u2, v.f0, v.f1, v.f2, v.l0,
-                                             v.l1, v.l2);
+                        apply_object_cell<P>(o, box_index(o, i, j, k), courant, u0, u1, u2, v.f0, v.f1, v.f2, none,
+                                             none, none);
                 }
             }
             // auxiliaries, then their corrections in boundary order (of a layer
@@ -541,33 +468,38 @@ __device__ __forceinline__ void flat_march(const GridK &g, const double *__restr
             flat_psi<P>(Y, qy, yx, yz);
             flat_psi<P>(W, qw, zy, zx);
             if (g.lay_order == kOrderXYZ) {
-                if (hx) pml_correct<P, IS_E>(v.f1, v.l1, v.m1, -qx.p0);
-                if (hx) pml_correct<P, IS_E>(v.f2, v.l2, v.m2, qx.p1);
-                if (hy) pml_correct<P, IS_E>(v.f2, v.l2, v.m2, -qy.p0);
-                if (hy) pml_correct<P, IS_E>(v.f0, v.l0, v.m0, qy.p1);
-                if (hw) pml_correct<P, IS_E>(v.f0, v.l0, v.m0, -qw.p0);
-                if (hw) pml_correct<P, IS_E>(v.f1, v.l1, v.m1, qw.p1);
+                if (hx) pml_correct<P, IS_E>(v.f1, none, v.m1, -qx.p0);
+                if (hx) pml_correct<P, IS_E>(v.f2, none, v.m2, qx.p1);
+                if (hy) pml_correct<P, IS_E>(v.f2, none, v.m2, -qy.p0);
+                if (hy) pml_correct<P, IS_E>(v.f0, none, v.m0, qy.p1);
+                if (hw) pml_correct<P, IS_E>(v.f0, none, v.m0, -qw.p0);
+                if (hw) pml_correct<P, IS_E>(v.f1, none, v.m1, qw.p1);
             } else {
 #pragma unroll 1
                 for (int o = flat_order(g, i, j, k), r = 0; r < 3; ++r, o >>= 4) {
                     if ((o & 15) == 0 && hx) {
-                        pml_correct<P, IS_E>(v.f1, v.l1, v.m1, -qx.p0);
-                        pml_correct<P, IS_E>(v.f2, v.l2, v.m2, qx.p1);
+                        pml_correct<P, IS_E>(v.f1, none, v.m1, -qx.p0);
+                        pml_correct<P, IS_E>(v.f2, none, v.m2, qx.p1);
                     } else if ((o & 15) == 1 && hy) {
-                        pml_correct<P, IS_E>(v.f2, v.l2, v.m2, -qy.p0);
-                        pml_correct<P, IS_E>(v.f0, v.l0, v.m0, qy.p1);
+                        pml_correct<P, IS_E>(v.f2, none, v.m2, -qy.p0);
+                        pml_correct<P, IS_E>(v.f0, none, v.m0, qy.p1);
                     } else if ((o & 15) == 2 && hw) {
-                        pml_correct<P, IS_E>(v.f0, v.l0, v.m0, -qw.p0);
-                        pml_correct<P, IS_E>(v.f1, v.l1, v.m1, qw.p1);
+                        pml_correct<P, IS_E>(v.f0, none, v.m0, -qw.p0);
+                        pml_correct<P, IS_E>(v.f1, none, v.m1, qw.p1);
                     }
                 }
             }
             for (unsigned sm = smask; sm; sm &= sm - 1) {
                 const ItemK &o = src.item[__ffs(sm) - 1];
-                if (i >= o.lo[0] && i < o.hi[0]) flat_source<P>(o, ny, nz, wave, i, j, k, v);
+                if (i < o.lo[0] || i >= o.hi[0]) continue;
+                T x = o.comp == 0 ? v.f0 : (o.comp == 1 ? v.f1 : v.f2);
+                flat_source<P>(o, ny, nz, wave, i, j, k, x);
+                if (o.comp == 0) v.f0 = x;
+                else if (o.comp == 1) v.f1 = x;
+                else v.f2 = x;
             }
-            flat_store<P>(v, s, listed == 0, 0);
-            flat_next<P, MAT>(s, v, step, istep);
+            flat_store(v, s, 0);
+            flat_next<T, MAT>(s, v, step, istep);
             X.q += istep;
             if (hy) Y.q += ystep;
             if (hw) W.q += wstep;
@@ -576,15 +508,14 @@ __device__ __forceinline__ void flat_march(const GridK &g, const double *__restr
     }
     if (listed > 0) {
         const int *idx = (IS_E ? g.srcE_idx : g.srcH_idx) + (IS_E ? g.srcE_off : g.srcH_off)[chunk];
-        flat_sources<P>(g, idx, listed, wave, xa, xb, j, k, jk, (T *)(IS_E ? g.E : g.H),
-                        (T *)(IS_E ? g.Elo : g.Hlo));
+        flat_sources<P>(g, idx, listed, wave, xa, xb, j, k, jk, (T *)(IS_E ? g.E : g.H));
     }
 }
 
 // Block b of a half step: chunk b mod n of the plane, x chunk b / n.  MAT: how
 // the material is read.
 template <class P, bool IS_E, int MAT>
-__global__ void __launch_bounds__(kFlatBlock, FlatTune<P>::blocks)
+__global__ void __launch_bounds__(kFlatBlock, kFlatBlocks)
     k_flat(const __grid_constant__ GridK g, const double *__restrict__ wave) {
     const unsigned n = g.flat_chunks, xc = blockIdx.x / n, chunk = blockIdx.x - xc * n;
     const int xa = g.ox + (int)xc * g.XC, xb = min(g.ex, xa + g.XC);
