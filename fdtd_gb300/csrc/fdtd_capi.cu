@@ -7,6 +7,7 @@
 #include <mutex>
 #include <vector>
 
+#include "fdtd_groups.hpp"
 #include "fdtd_kernels.cuh"
 #include "fdtd_persistent.cuh"
 #include "fdtd_plan.hpp"
@@ -914,56 +915,79 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
     }
 
     // what the fused passes apply, in order: the objects, and per half step the
-    // sources, an E source of several soft points as one group (kItemSoftGroup)
+    // sources, the soft points of an E source in groups (kItemSoftGroup): one
+    // for the flat passes, which look for a column's points once, else as many
+    // as it takes to keep their boxes filled (fdtd_groups.hpp)
     struct Group {
         int item;
-        std::vector<long long> cells;  // empty: the box is full
+        std::vector<long long> cells;  // flat passes: empty where the box is full
+        std::vector<int> first;        // the others
         std::vector<double> weights;
         size_t at_cells, at_weights;
     };
     std::vector<Group> groups;
     std::vector<int> use_obj, use_src[2];
     for (int q = 0; q < srcE0; ++q) use_obj.push_back(q);
-    for (int side = 0; side < 2; ++side) {
+    auto group_points = [&](int first, int last, bool by_column) {  // returns the item
+        std::vector<int> at(last - first);
+        for (int r = first; r < last; ++r) at[r - first] = r;
+        auto column = [&](int r) {
+            return ((long long)items[r].lo[1] * d->nz + items[r].lo[2]) * d->nx + items[r].lo[0];
+        };
+        ItemK it = items[first];
+        it.kind = kItemSoftGroup;
+        it.aux = last - first;
+        bool full = true;  // n distinct cells (they are sorted) in a box of n cells fill it, in box order
+        for (int r = first; r < last; ++r) {
+            for (int a = 0; a < 3; ++a) {
+                it.lo[a] = std::min(it.lo[a], items[r].lo[a]);
+                it.hi[a] = std::max(it.hi[a], items[r].hi[a]);
+            }
+            full = full && (r == first || column(r) != column(r - 1));
+        }
+        it.bny = it.hi[1] - it.lo[1];
+        it.bnz = it.hi[2] - it.lo[2];
+        const long long box = (long long)(it.hi[0] - it.lo[0]) * it.bny * it.bnz;
+        full = full && box == last - first;
+        if (by_column && !full)
+            std::stable_sort(at.begin(), at.end(), [&](int x, int y) { return column(x) < column(y); });
+        Group gr;
+        for (int r : at) {
+            if (by_column && !full) gr.cells.push_back(column(r));
+            gr.weights.push_back(items[r].weight);
+        }
+        if (!by_column && !full) {
+            gr.first.assign((size_t)box + 1, 0);
+            for (int r : at) gr.first[box_index(it, items[r].lo[0], items[r].lo[1], items[r].lo[2]) + 1]++;
+            for (size_t c = 1; c < gr.first.size(); ++c) gr.first[c] += gr.first[c - 1];
+        }
+        gr.item = (int)items.size();
+        items.push_back(it);
+        groups.push_back(gr);
+        return gr.item;
+    };
+    auto source_items = [&](int side, bool by_column) {
+        std::vector<int> use;
         const int first = side == 0 ? srcE0 : srcH0;
         const int last = first + (side == 0 ? d->n_sources_E : d->n_sources_H);
         int e;
         for (int q = first; q < last; q = e) {
             e = q + 1;
             while (e < last && items[e].source == items[q].source) ++e;
-            bool one = side == 0 && e - q > 1;
+            bool soft = side == 0;
             for (int r = q; r < e; ++r)
-                one = one && items[r].kind == FDTD_ITEM_SOFT && items[r].comp == items[q].comp &&
-                      items[r].column == items[q].column;
-            if (!one) {
-                for (int r = q; r < e; ++r) use_src[side].push_back(r);
-                continue;
+                soft = soft && items[r].kind == FDTD_ITEM_SOFT && items[r].comp == items[q].comp &&
+                       items[r].column == items[q].column;
+            for (int r = q, re; r < e; r = re) {
+                re = !soft       ? r + 1
+                     : by_column ? e
+                                 : group_end(r, e, [&](int x, int a) { return items[x].lo[a]; });
+                use.push_back(re - r > 1 ? group_points(r, re, by_column) : r);
             }
-            Group gr;
-            ItemK it = items[q];
-            it.kind = kItemSoftGroup;
-            it.aux = e - q;
-            for (int r = q; r < e; ++r) {
-                for (int a = 0; a < 3; ++a) {
-                    it.lo[a] = std::min(it.lo[a], items[r].lo[a]);
-                    it.hi[a] = std::max(it.hi[a], items[r].hi[a]);
-                }
-                gr.cells.push_back(((long long)items[r].lo[0] * d->ny + items[r].lo[1]) * d->nz + items[r].lo[2]);
-                gr.weights.push_back(items[r].weight);
-            }
-            it.bny = it.hi[1] - it.lo[1];
-            it.bnz = it.hi[2] - it.lo[2];
-            // n distinct cells (they are sorted) in a box of n cells fill it, in box order
-            bool full = (long long)(it.hi[0] - it.lo[0]) * it.bny * it.bnz == (long long)gr.cells.size();
-            for (size_t r = 1; r < gr.cells.size(); ++r) full = full && gr.cells[r] != gr.cells[r - 1];
-            if (full) gr.cells.clear();
-            gr.item = (int)items.size();
-            use_src[side].push_back(gr.item);
-            items.push_back(it);
-            groups.push_back(gr);
         }
-    }
-    const int ndev_items = (int)items.size();
+        return use;
+    };
+    for (int side = 0; side < 2; ++side) use_src[side] = source_items(side, flat);
 
     std::vector<int> obj_off, obj_idx, se_off, se_idx, sh_off, sh_idx;
     if (!flat) {
@@ -1273,7 +1297,7 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
                     p.onepass = 1;
                     p.onepass_hcopy = per_x ? 1 : 0;
                     build_csr(to, items, use_obj, oo_off, oo_idx, true);
-                    build_csr(to, items, use_src[0], ose_off, ose_idx, true);
+                    build_csr(to, items, flat ? source_items(0, false) : use_src[0], ose_off, ose_idx, true);
                     build_csr(to, items, use_src[1], osh_off, osh_idx, true);
                 } else {
                     p.onepass_why = 9;
@@ -1301,6 +1325,7 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
 
     // one device allocation for the plan's tables
     auto align = [](size_t v) { return (v + 255) & ~(size_t)255; };
+    const int ndev_items = (int)items.size();
     const size_t b_items = align(sizeof(ItemK) * std::max(1, ndev_items));
     const size_t b_lists = align(sizeof(int) * (obj_off.size() + obj_idx.size() + se_off.size() + se_idx.size() +
                                                 sh_off.size() + sh_idx.size() + oo_off.size() + oo_idx.size() +
@@ -1311,8 +1336,8 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
     size_t b_groups = 0;
     for (Group &gr : groups) {
         gr.at_cells = b_items + b_lists + b_runs + b_status + b_groups;
-        gr.at_weights = gr.at_cells + sizeof(long long) * gr.cells.size();
-        b_groups += sizeof(long long) * gr.cells.size() + sizeof(double) * gr.weights.size();
+        gr.at_weights = gr.at_cells + sizeof(long long) * gr.cells.size() + (sizeof(int) * gr.first.size() + 7) / 8 * 8;
+        b_groups = gr.at_weights + sizeof(double) * gr.weights.size() - (b_items + b_lists + b_runs + b_status);
     }
     std::vector<char> host(b_items + b_lists + b_runs + b_status + b_groups, 0);
     int *lists = (int *)(host.data() + b_items);
@@ -1347,7 +1372,9 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
         if (!gr.cells.empty())
             memcpy(host.data() + gr.at_cells, gr.cells.data(), sizeof(long long) * gr.cells.size());
         memcpy(host.data() + gr.at_weights, gr.weights.data(), sizeof(double) * gr.weights.size());
-        items[gr.item].coef[0] = gr.cells.empty() ? nullptr : (const char *)p.dev_mem + gr.at_cells;
+        if (!gr.first.empty()) memcpy(host.data() + gr.at_cells, gr.first.data(), sizeof(int) * gr.first.size());
+        const bool full = gr.cells.empty() && gr.first.empty();
+        items[gr.item].coef[0] = full ? nullptr : (const char *)p.dev_mem + gr.at_cells;
         items[gr.item].coef[1] = (const char *)p.dev_mem + gr.at_weights;
     }
     if (ndev_items) memcpy(host.data(), items.data(), sizeof(ItemK) * ndev_items);
@@ -1355,6 +1382,8 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
         FlatSources &f = side == 0 ? g.src_E : g.src_H;
         const std::vector<int> &use = use_src[side];
         f.n = use.size() <= kFlatSources ? (int)use.size() : -1;
+        for (const Group &gr : groups)  // points that a column has to look for
+            if (!gr.cells.empty() && std::find(use.begin(), use.end(), gr.item) != use.end()) f.n = -1;
         if (!(side == 0 ? g.fuse_src_E : g.fuse_src_H)) f.n = 0;  // in kernels of their own
         for (int q = 0; q < f.n; ++q) f.item[q] = items[use[q]];
     }

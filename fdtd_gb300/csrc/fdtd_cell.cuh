@@ -186,32 +186,15 @@ __device__ __forceinline__ void apply_objects_v(const GridK &g, int i, int j, in
     }
 }
 
-// The points [a, b) of a soft source on cell (i, j, k) of its bounding box (a
-// cell may be listed more than once): its place in a box that is full, else
-// found by bisection.
+// The points [a, b) of a group on cell (i, j, k) of its box (a cell may be
+// listed more than once), by its place in the box.
 struct SoftSpan {
     int a, b;
 };
-__device__ __forceinline__ SoftSpan soft_span(const ItemK &s, int ny, int nz, int i, int j, int k) {
-    const long long *cells = (const long long *)s.coef[0];
-    if (cells == nullptr) {
-        const int a = (int)box_index(s, i, j, k);
-        return SoftSpan{a, a + 1};
-    }
-    const long long cell = ((long long)i * ny + j) * nz + k;
-    int a = 0, n = s.aux;
-    while (n > 0) {
-        const int h = n >> 1;
-        if (cells[a + h] < cell) {
-            a += h + 1;
-            n -= h + 1;
-        } else {
-            n = h;
-        }
-    }
-    int b = a;
-    while (b < s.aux && cells[b] == cell) ++b;
-    return SoftSpan{a, b};
+__device__ __forceinline__ SoftSpan soft_span(const ItemK &s, int i, int j, int k) {
+    const int at = (int)box_index(s, i, j, k);
+    const int *first = (const int *)s.coef[0];
+    return first == nullptr ? SoftSpan{at, at + 1} : SoftSpan{first[at], first[at + 1]};
 }
 
 // Sources of one cell (fdtd/sources.py:93-109, 278-297, 476-486), in order.
@@ -233,7 +216,7 @@ __device__ __forceinline__ void apply_sources(const GridK &g, const int *idx, co
             const double *wt = &s.weight;
             SoftSpan q{0, 1};
             if (GROUPS && s.kind == kItemSoftGroup) {
-                q = soft_span(s, g.ny, g.nz, i, j, k);
+                q = soft_span(s, i, j, k);
                 wt = (const double *)s.coef[1];
             }
 #pragma unroll 1

@@ -42,12 +42,14 @@ struct ItemK {
     int aux;  // FDTD_ITEM_FEEDBACK: its point in the current-probe list; kItemSoftGroup: its points
 };
 
-// All points of one soft source as one item of the fused passes: lo/hi their
-// bounding box, coef[0] their linear cells in ascending order (null: every
-// cell of the box exactly once, in box order), coef[1] their weights (double),
-// aux their number.  A line source of n points as n items had every thread of
-// its tiles test n boxes per plane: 2D 1500x1100 float32, a line of 550 cells,
-// 489 us per step against 41.7.
+// Points of one soft source as one item of the fused passes: lo/hi their
+// bounding box, coef[1] their weights (double), aux their number.  coef[0] is
+// null where they are the cells of the box, each once, in box order.  Else it
+// holds, for the flat passes, their cells by column ((j nz + k) nx + i, long
+// long, ascending); for the others, the first point of every cell of the box
+// and their number at the end (int).  A line source of n points as n items had
+// every thread of its tiles test n boxes per plane: 2D 1500x1100 float32, a
+// line of 550 cells, 489 us per step against 41.7.
 constexpr int kItemSoftGroup = 100;
 
 // Material modes of a staged pass: the inverse material read per cell as
@@ -62,7 +64,7 @@ constexpr int MAT_FULL = 0, MAT_IDS = 1, MAT_UNIFORM = 2;
 // H half 195 -> 175).
 constexpr int kFlatSources = 4;
 struct FlatSources {
-    int n;  // -1: more than kFlatSources, the chunk lists are used
+    int n;  // -1: more than kFlatSources, or points in a box not full: the chunk lists are used
     ItemK item[kFlatSources];
 };
 
@@ -361,7 +363,7 @@ __device__ __forceinline__ bool in_box(const ItemK &it, int i, int j, int k) {
            k < it.hi[2];
 }
 
-__device__ __forceinline__ size_t box_index(const ItemK &it, int i, int j, int k) {
+__host__ __device__ __forceinline__ size_t box_index(const ItemK &it, int i, int j, int k) {
     return ((size_t)(i - it.lo[0]) * it.bny + (j - it.lo[1])) * it.bnz + (k - it.lo[2]);
 }
 

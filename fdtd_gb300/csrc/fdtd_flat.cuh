@@ -78,11 +78,30 @@ __device__ __forceinline__ FlatPlace flat_place(const GridK &g, unsigned chunk) 
     return p;
 }
 
+// First point of a group at or after key (its cells by column, ascending).
+__device__ __forceinline__ int point_at(const ItemK &s, long long key) {
+    const long long *cells = (const long long *)s.coef[0];
+    int a = 0, n = s.aux;
+    while (n > 0) {
+        const int h = n >> 1;
+        if (cells[a + h] < key) {
+            a += h + 1;
+            n -= h + 1;
+        } else {
+            n = h;
+        }
+    }
+    return a;
+}
+
 // The chunk's listed sources (where the kernel's parameters do not hold them) on
 // planes [xa, xb), after the march has stored those planes: one source after
 // the other over the planes (each cell gets them in order), so that a thread
-// looks at a source once and not once a plane: 128^3 with 40 points 68 -> 46 us
-// per step, with 200 points 118 -> 76.
+// looks at a source once and not once a plane, and finds its column's first
+// point in a group by one bisection.  us per step, plane by plane and with a
+// bisection per plane inside the march, and now: 128^3 with 40 points 68 -> 46,
+// 200 points 118 -> 76; 2D 1500x1100 with a diagonal line 74 -> 33, 128^3 62 ->
+// 39, with six of them 355 -> 54.
 // Not inlined: the march would lose the registers (192x192x96 E half and H half
 // 84 -> 75, 131x150x97 in the persistent loop 53.5 -> 50.6).
 template <class P, bool IS_E>
@@ -91,7 +110,7 @@ __device__ __noinline__ void flat_listed(const GridK &g, const double *__restric
     using T = typename P::T;
     const FlatPlace pl = flat_place(g, chunk);
     if (!pl.in) return;
-    const int ny = g.ny, nz = g.nz, j = pl.j, k = pl.k;
+    const int nx = g.nx, ny = g.ny, nz = g.nz, j = pl.j, k = pl.k;
     const long nyz = (long)ny * nz, jk = (long)j * nz + k;
     T *F = (T *)(IS_E ? g.E : g.H);
     const int *off = IS_E ? g.srcE_off : g.srcH_off, *idx = IS_E ? g.srcE_idx : g.srcH_idx;
@@ -105,11 +124,17 @@ __device__ __noinline__ void flat_listed(const GridK &g, const double *__restric
         T *f = F + 3 * jk + s.comp;
         const T wv = (T)wave[s.column];
         if (IS_E && s.kind == kItemSoftGroup) {
+            const long long *cells = (const long long *)s.coef[0];
             const double *weights = (const double *)s.coef[1];
+            if (cells == nullptr) {
 #pragma unroll 1
-            for (int i = i0; i < end; ++i) {
-                const SoftSpan q = soft_span(s, ny, nz, i, j, k);
-                for (int a = q.a; a < q.b; ++a) P::add_prod(f[3 * (i * nyz)], none, (T)weights[a], wv);
+                for (int i = i0; i < end; ++i)
+                    P::add_prod(f[3 * (i * nyz)], none, (T)weights[box_index(s, i, j, k)], wv);
+            } else {
+                const long long key = (long long)jk * nx;
+#pragma unroll 1
+                for (int a = point_at(s, key + i0); a < s.aux && cells[a] < key + end; ++a)
+                    P::add_prod(f[3 * ((cells[a] - key) * nyz)], none, (T)weights[a], wv);
             }
         } else {
             const bool soft = s.kind == FDTD_ITEM_SOFT;
@@ -497,14 +522,10 @@ __device__ __forceinline__ void flat_march(const GridK &g, const double *__restr
                 if (i < o.lo[0] || i >= o.hi[0]) continue;
                 T x = o.comp == 0 ? v.f0 : (o.comp == 1 ? v.f1 : v.f2);
                 const T wv = (T)wave[o.column];
-                if (IS_E && o.kind == kItemSoftGroup) {
-                    const SoftSpan q = soft_span(o, ny, nz, i, j, k);
-                    for (int a = q.a; a < q.b; ++a) P::add_prod(x, none, (T)((const double *)o.coef[1])[a], wv);
-                } else if (o.kind == FDTD_ITEM_SOFT) {
-                    P::add_prod(x, none, (T)o.weight, wv);
-                } else {
-                    P::set(x, none, P::mul((T)o.weight, wv));
-                }
+                if (IS_E && o.kind == kItemSoftGroup)  // (its box is full)
+                    P::add_prod(x, none, (T)((const double *)o.coef[1])[box_index(o, i, j, k)], wv);
+                else if (o.kind == FDTD_ITEM_SOFT) P::add_prod(x, none, (T)o.weight, wv);
+                else P::set(x, none, P::mul((T)o.weight, wv));
                 if (o.comp == 0) v.f0 = x;
                 else if (o.comp == 1) v.f1 = x;
                 else v.f2 = x;
