@@ -37,6 +37,7 @@ static bool aligned8(const void *ptr) { return ((uintptr_t)ptr & 7u) == 0; }
 
 // Cells from which a thick shell is split off automatically (see mode 4 below).
 static const long kPartition32 = 3800000, kPartition32odd = 2600000, kPartition64 = 500000, kPartition32c = 800000;
+static const long kPartition64fit = 1L << 20, kPartition32cfit = 1300000;  // rows that fill the register tiles
 
 // Threads along z of a register-streaming tile for zt threads' worth of
 // cells: the next power of two up to 32, or 16 where that pads less (config 5,
@@ -375,7 +376,15 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
     // 2.9M 114 vs 91; float64 (register tiles) 0.26M 58 vs 68, 0.6M 107 vs 97,
     // 1.1M 209 vs 159, 2.1M 300 vs 255, 5.1M 524 vs 491, 6.9M 770 vs 628;
     // float32c 0.26M 20 vs 31, 1.1M 70 vs 58, 1.9M 104 vs 82, 5.7M 225 vs 186,
-    // 30M odd rows, 10 %, 902 vs 822.
+    // 30M odd rows, 10 %, 902 vs 822.  Rows that fill the fused register tiles
+    // to the last thread (nz = 64, 96, 128, 256) leave the partition less to
+    // gain, and it starts later, at 2^20 cells in float64 and 1.3M in float32c:
+    // float64 64x64x128 80 vs 84, 96x96x64 91 vs 103, 96^3 118 vs 127,
+    // 104x104x96 135 vs 142, from there 128x128x64 144 vs 145, 64x128x128 149
+    // vs 141, 96x96x128 166 vs 149, 112x112x96 152 vs 156, 128^3 280 vs 242;
+    // rows that do not, 100x100x80 127 vs 116, 90x90x72 114 vs 104; float32c
+    // 112x112x64 37.5 vs 42.9, 128x128x64 45.1 vs 49.6, 96x96x128 48.7 vs 50.8,
+    // from there 96x112x128 56.7 vs 54.9, 128^3 83.7 vs 77.6.
     // cells per shell thread along z: two floats where rows are even, else one
     p.shell_v = d->precision == FDTD_FLOAT64 || d->nz % 2 != 0 || !aligned8(d->E) || !aligned8(d->H) ||
                         !aligned8(d->inv_eps) || !aligned8(d->inv_mu) ||
@@ -412,8 +421,10 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
         const bool ok = g.nslab > 0 && !slab_after_periodic && (vec || d->nz > 1) && inner;
         if (pml_base == 4 && !(ok && vec)) return FDTD_ERR_UNSUPPORTED;
         bool want = ok && pml_base == 4;
-        const long from = d->precision == FDTD_FLOAT64 ? kPartition64
-                          : d->precision == FDTD_FLOAT32C ? kPartition32c
+        const int zt = d->nz / vmax;
+        const bool fit = vec && zt % tile_width(zt) == 0;
+        const long from = d->precision == FDTD_FLOAT64    ? (fit ? kPartition64fit : kPartition64)
+                          : d->precision == FDTD_FLOAT32C ? (fit ? kPartition32cfit : kPartition32c)
                           : vec                           ? kPartition32 : kPartition32odd;
         if (ok && pml_base == 0 && d->persistent != 2 && ncell >= from) {
             // float64 (arithmetic bound, register-streaming interior) from a

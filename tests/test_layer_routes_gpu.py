@@ -108,3 +108,18 @@ def test_layers_of_one_axis_that_share_cells(fd, spec, shape):
         f = _run(fd, shape, spec, **tune)
         assert f._engine.tiling()["persistent"] == (tune.get("persistent") == 2)
         assert torch.equal(f.E, g.E) and torch.equal(f.H, g.H), tune
+
+
+@pytest.mark.parametrize("prec,shape,split", [
+    ("float64", (96, 96, 96), 0), ("float64", (96, 96, 64), 0), ("float64", (128, 128, 64), 2),
+    ("float64", (100, 100, 80), 2), ("float32c", (112, 112, 64), 0), ("float32c", (96, 112, 128), 2),
+    ("float32c", (104, 104, 104), 2),
+])
+def test_partition_where_rows_fill_the_tiles(fd, prec, shape, split):
+    """Rows that fill the register tiles to the last thread keep mid-sized grids
+    in the persistent loop; the partition starts at more cells."""
+    fd.set_backend("gb300." + prec)
+    g = fd.Grid(shape, grid_spacing=155e-9)
+    _layers(fd, g, [(a, h, 10) for a in range(3) for h in range(2)])
+    t = g._ensure_engine().tiling()
+    assert t["pml_split"] == split and t["persistent"] == (split == 0)
