@@ -2,6 +2,7 @@
 // descriptor validation, launch tiling, per-CTA object/source lists and
 // dispatch to the per-precision launch sequences.
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -461,13 +462,26 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
     // CTAs that hold them late, and their auxiliary rows enlarge every stage.
     // The automatic choice therefore keeps only leading y slabs, for float32
     // with compact materials.
-    // 2D grids (nz = 1) of 8M cells and more split too, but for the flat half
-    // steps of float32 (4000^2, us per step: flat 275, split 332)
+    // Flat half steps for float32, but for large 2D grids of several materials
+    // (few cells of a plane are in layers there, and the 40 registers of the
+    // register tiles keep more warps on the loads).  us per step, flat vs
+    // register: 1186x3541 one material 94 vs 99, blocks 120 vs 106, with an
+    // object 121 vs 106; 3000^2 219 vs 205; in the persistent loop with an
+    // object 700x900 24 vs 24, 1100^2 38 vs 35, 1900x1500 91 vs 68, blocks
+    // alone 1100^2 28 vs 35, 1500x1100 34 vs 42, 1900x1500 68 vs 65.
+    const bool flat2d = d->nz > 1 || (mat_want[0] == MAT_UNIFORM && mat_want[1] == MAT_UNIFORM) ||
+                        ncell < (d->n_objects > 0 ? 1200000 : 2500000);
+    // 2D grids (nz = 1) of 8M cells and more split too, in float32 only the
+    // register tiles and from 16M cells.  us per step, fused vs split: flat
+    // 4000^2 233 vs 268, 8192^2 846 vs 880; register 4000x2200 194 vs 205,
+    // 3500^2 252 vs 258, 4000^2 320 vs 307, 5500^2 540 vs 515, 8192^2 1040 vs 986.
+    GridK all = g;
+    const long split2d = d->precision != FDTD_FLOAT32               ? 8L << 20
+                         : flat2d && flat_layers(all, 2 * esize) ? LONG_MAX : 16000000L;
     p.pml_split = g.nslab > 0 && p.n_shell == 0 &&
                   (pml_base >= 2 ||
-                   (pml_base == 0 && ncell >= (8L << 20) &&
-                    ((vec && (long)d->nz * 3 * (long)esize >= 768) ||
-                     (d->nz == 1 && d->precision != FDTD_FLOAT32))));
+                   (pml_base == 0 && ((ncell >= (8L << 20) && vec && (long)d->nz * 3 * (long)esize >= 768) ||
+                                      (d->nz == 1 && ncell >= split2d))));
     int kfs = 0;  // leading slabs kept in the fused pass when split
     const bool auto_keep = pml_base == 0 && d->precision == FDTD_FLOAT32 && mat_want[0] != MAT_FULL &&
                            mat_want[1] != MAT_FULL;
@@ -679,15 +693,6 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
     g.nlut_H = g.mat_H == MAT_FULL ? 0 : d->n_mu_table;
     g.mid_E = g.mat_E == MAT_IDS ? d->eps_index : nullptr;
     g.mid_H = g.mat_H == MAT_IDS ? d->mu_index : nullptr;
-    // Flat half steps for float32, but for large 2D grids of several materials
-    // (few cells of a plane are in layers there, and the 40 registers of the
-    // register tiles keep more warps on the loads).  us per step, flat vs
-    // register: 1186x3541 one material 94 vs 99, blocks 120 vs 106, with an
-    // object 121 vs 106; 3000^2 219 vs 205; in the persistent loop with an
-    // object 700x900 24 vs 24, 1100^2 38 vs 35, 1900x1500 91 vs 68, blocks
-    // alone 1100^2 28 vs 35, 1500x1100 34 vs 42, 1900x1500 68 vs 65.
-    const bool flat2d = d->nz > 1 || (g.mat_E == MAT_UNIFORM && g.mat_H == MAT_UNIFORM) ||
-                        ncell < (d->n_objects > 0 ? 1200000 : 2500000);
     // Layers that the flat passes do not take (flat_layers) keep the register
     // tiles, which stay in the persistent loop.  us per step, a general flat
     // form (one launch per half step) vs register: layers of one axis that

@@ -123,3 +123,19 @@ def test_partition_where_rows_fill_the_tiles(fd, prec, shape, split):
     _layers(fd, g, [(a, h, 10) for a in range(3) for h in range(2)])
     t = g._ensure_engine().tiling()
     assert t["pml_split"] == split and t["persistent"] == (split == 0)
+
+
+@pytest.mark.parametrize("shape,several,split", [((4000, 4000, 1), True, 1), ((4000, 4000, 1), False, 0),
+                                                 ((3500, 3500, 1), True, 0)])
+def test_layers_of_large_2d_grids(fd, shape, several, split):
+    """The layers of large 2D float32 grids in kernels of their own: where the
+    grid runs register tiles (several materials), not flat ones."""
+    fd.set_backend("gb300.float32")
+    eps = 1.0
+    if several:
+        eps = np.ones(shape)
+        eps[500:900, 300:800] = 4.0
+        eps[1500:1700, 800:1100] = 2.25
+    g = fd.Grid(shape, grid_spacing=155e-9, permittivity=eps)
+    _layers(fd, g, [(0, 0, 16), (0, 1, 16), (1, 0, 16), (1, 1, 16)])
+    assert g._ensure_engine().tiling()["pml_split"] == split
