@@ -526,14 +526,18 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
     bool fused_z = false;  // a z slab inside the fused pass (divergent warps)
     for (int s = 0; s < ks; ++s) fused_z |= g.slab[s].axis == 2;
     // a partition's interior: the staged pass for float32 with compact
-    // materials on both passes from 24M cells, else the register-streaming one
-    // (config 2, full permittivity, 0.375 vs 0.494 ms per step; config 5
-    // float64 2.49 vs 2.57, float32c 0.85 vs 0.95; float32 with compact
-    // materials, staged vs register, us per step: 16.8M cells 413 vs 370,
-    // 18.5M 410 vs 373, 24.2M 518 vs 491, 24.6M 466 vs 482, 28M 558 vs 582,
-    // 64M 1072 vs 1166, 87M 1582 vs 1658)
+    // materials on both passes, from 24M cells where both are uniform and from
+    // 14M where one is indexed (which the register tiles read in full), else
+    // the register-streaming one (config 2, full permittivity, 0.375 vs 0.494
+    // ms per step; config 5 float64 2.49 vs 2.57, float32c 0.85 vs 0.95).  us
+    // per step, register vs staged: uniform 12.9M cells 239 vs 254, 16.8M 278
+    // vs 282, 18.9M 312 vs 313, 22.0M 368 vs 366, 23.9M 385 vs 389, 24.5M 443 vs
+    // 445, 26.2M 461 vs 450, 28.3M 509 vs 496; indexed 11.2M 227 vs 227, 12.9M
+    // 255 vs 262, 14.7M 288 vs 282, 17.8M 335 vs 322, 21.0M 402 vs 396, 23.2M
+    // 422 vs 399, 25.2M 451 vs 422.
+    const bool indexed = mat_want[0] == MAT_IDS || mat_want[1] == MAT_IDS;
     const bool shell_tma = d->precision == FDTD_FLOAT32 && mat_want[0] != MAT_FULL && mat_want[1] != MAT_FULL &&
-                           ncell >= 24000000;
+                           ncell >= (indexed ? 14000000 : 24000000);
     const bool tma = d->variant == 2 || (d->variant == 0 && vec && !fused_z && (long)bnz * 3 * (long)esize >= 768 &&
                                          (p.n_shell == 0 || shell_tma));
     Tiling t{};

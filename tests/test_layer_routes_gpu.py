@@ -139,3 +139,21 @@ def test_layers_of_large_2d_grids(fd, shape, several, split):
     g = fd.Grid(shape, grid_spacing=155e-9, permittivity=eps)
     _layers(fd, g, [(0, 0, 16), (0, 1, 16), (1, 0, 16), (1, 1, 16)])
     assert g._ensure_engine().tiling()["pml_split"] == split
+
+
+@pytest.mark.parametrize("shape,several,staged", [((256, 240, 240), True, True), ((256, 240, 240), False, False),
+                                                  ((224, 224, 224), True, False)])
+def test_interior_of_a_partition(fd, shape, several, staged):
+    """The interior of a float32 partition runs staged where the material is
+    indexed (the register tiles read it in full) at fewer cells than where it
+    is uniform."""
+    fd.set_backend("gb300.float32")
+    eps = 1.0
+    if several:
+        eps = np.ones(shape)
+        eps[50:90, 30:80, 20:100] = 4.0
+        eps[150:170, 80:110, 60:190] = 2.25
+    g = fd.Grid(shape, grid_spacing=155e-9, permittivity=eps)
+    _layers(fd, g, [(a, h, 14) for a in range(3) for h in range(2)])
+    t = g._ensure_engine().tiling()
+    assert t["pml_split"] == 2 and t["variant"] == (2 if staged else 1)
