@@ -731,7 +731,8 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
         // float32c 93 -> 83, 111x112x128 84 -> 82; 223x224x100 float32 186 ->
         // 154, 197x198x128 161 -> 151.
         const int zt = (bnz + t.V - 1) / t.V;
-        if (t.TZ == 32 && zt % 32 > 16 && zt % 16 <= 8 && zt % 16 != 0) {
+        // (The stages of a staged interior are laid out for the tile it has.)
+        if (!use_tma && t.TZ == 32 && zt % 32 > 16 && zt % 16 <= 8 && zt % 16 != 0) {
             t.TZ = 16;
             t.TY = kThreads / 16;
         }
