@@ -414,7 +414,8 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
         // Rows that do not divide into vectors (an odd nz, say) leave the
         // interior to one cell per thread, and their z faces need no alignment
         // but the shell threads' own.
-        const int za = !vec ? p.shell_v : (d->precision != FDTD_FLOAT64 ? 16 : 4);
+        const bool idx = d->variant == 2 && (mat_want[0] == MAT_IDS || mat_want[1] == MAT_IDS);
+        const int za = !vec ? p.shell_v : (idx || d->precision != FDTD_FLOAT64 ? 16 : 4);
         const int zu = vec ? vmax : p.shell_v;
         lo[2] = (lo[2] + za - 1) / za * za;
         hi[2] = hi[2] / zu * zu;
