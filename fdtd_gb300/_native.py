@@ -132,6 +132,7 @@ SIGNATURES = {
     "fdtd_plan_tiling": (c_int32, [c_void_p, ctypes.POINTER(c_int64)]),
     "fdtd_plan_step_fusion": (c_int32, [c_void_p, ctypes.POINTER(c_int32), ctypes.POINTER(c_int32),
                                         ctypes.POINTER(c_int32)]),
+    "fdtd_plan_materials": (c_int32, [c_void_p, ctypes.POINTER(c_int32), ctypes.POINTER(c_int32)]),
     "fdtd_status_string": (ctypes.c_char_p, [c_int32]),
     "fdtd_last_cuda_error": (c_int32, []),
     "fdtd_abi_sizeof": (ctypes.c_size_t, [c_int32]),

@@ -272,7 +272,7 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
     if (d->materials_scaled != 0 && d->materials_scaled != 1) return FDTD_ERR_ARGUMENT;
     if (d->materials_scaled && d->precision != FDTD_FLOAT64) return FDTD_ERR_UNSUPPORTED;
     g.scaled = d->materials_scaled;
-    // compact material copies: validated here, used only by the staged passes
+    // compact material copies, where given and usable
     int mat_want[2] = {MAT_FULL, MAT_FULL};
     {
         const void *tab[2] = {d->eps_table, d->mu_table};
@@ -1900,6 +1900,20 @@ int fdtd_plan_tiling(const fdtd_plan *plan, int64_t *out8) {
     out8[5] = p.persistent ? 1 : p.launches_per_step;  // persistent: one launch per fdtd_run call
     out8[6] = p.persistent ? 5 : p.variant + (p.pml_split ? 10 : 0) + (p.n_shell ? 20 : 0);
     out8[7] = p.k.stages;
+    return FDTD_OK;
+}
+
+int fdtd_plan_materials(const fdtd_plan *plan, int32_t *eps, int32_t *mu) {
+    if (!plan || !eps || !mu) return FDTD_ERR_ARGUMENT;
+    const Plan &p = plan->p;
+    *eps = p.onepass ? p.ko[0].mat_E : p.kf.mat_E;
+    *mu = p.onepass ? p.ko[0].mat_H : p.kf.mat_H;
+    if (p.onepass || p.variant == 2) return FDTD_OK;
+    // register tiles read an indexed material in full, and so does the H half
+    // of the persistent loop; its register tiles read any permittivity in full
+    if (!p.flat && *eps == MAT_IDS) *eps = MAT_FULL;
+    if ((!p.flat || p.persistent) && *mu == MAT_IDS) *mu = MAT_FULL;
+    if (!p.flat && p.persistent) *eps = MAT_FULL;
     return FDTD_OK;
 }
 

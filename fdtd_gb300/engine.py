@@ -10,10 +10,10 @@
   grid precision, grown geometrically; detectors view their slice of it;
 * DFT phases -- (n, n_freq_total, 2) float64 (cos, -sin) per step.
 
-* compact material copies -- for the staged passes, a table of the distinct
-  inverse-material value triples and a one-byte index per cell (or one triple
-  for a uniform material), kept in step with in-place changes of the
-  material arrays (``compact_material``).
+* compact material copies -- a table of the distinct inverse-material value
+  triples and a one-byte index per cell (or one triple for a uniform
+  material), kept in step with in-place changes of the material arrays that
+  torch counts (``compact_material``).
 
 The plan is rebuilt when components are registered, when an object's
 coefficients change, when the compact copies change layout, or when the
@@ -47,8 +47,7 @@ _MAX_TABLE = 256  # distinct value triples a one-byte material index can address
 
 
 def compact_material(x, chunk=1 << 25, index_ok=True):
-    """Compact copy of a (nx, ny, nz, 3) inverse-material array for the staged
-    passes: ``(table, index)`` with ``table`` an (n, 3) array of value triples
+    """Compact copy of a (nx, ny, nz, 3) inverse-material array: ``(table, index)`` with ``table`` an (n, 3) array of value triples
     and ``index`` the uint8 (nx, ny, nz) table row of every cell, or
     ``(table, None)`` when every cell holds the same triple; ``None`` when the
     cells hold more than 256 distinct triples, or more than one and
@@ -233,7 +232,7 @@ class Engine:
         self.grid = grid
         self.x_chunk = x_chunk
         # fused-pass kernel choice: variant 0 auto / 1 flat or register streaming / 2 TMA-staged
-        # materials: 0 compact copies for the staged passes where possible, 1 full arrays only
+        # materials: 0 compact copies where possible, 1 full arrays only
         # step_fusion: 0 auto / 1 two passes per step / 2 one pass per step (where allowed)
         # persistent: 0 auto / 1 one launch per half step / 2 one persistent launch per run() (where allowed)
         self.tuning = {"variant": 0, "tile_rows": 0, "stages": 0, "pml_mode": 0, "materials": 0, "step_fusion": 0,
@@ -333,13 +332,16 @@ class Engine:
         return rebuild
 
     def compact_materials(self):
-        """How the plan's staged passes read each material (inverse permittivity,
-        inverse permeability): None (full arrays; always for the register
-        kernels), ("uniform", 1) or ("index", n distinct value triples)."""
-        if self.plan is None or self.tiling()["variant"] not in (2, 4):
+        """How the plan's half steps read each material (inverse permittivity,
+        inverse permeability): None (full arrays), ("uniform", 1) or ("index",
+        rows of the table)."""
+        if self.plan is None:
             return [None, None]
-        return [None if e is None else (("index", e[0].shape[0]) if e[1] is not None else ("uniform", 1))
-                for e in self._compact]
+        eps, mu = ctypes.c_int32(0), ctypes.c_int32(0)
+        _native.check(_native.load().fdtd_plan_materials(self.plan, ctypes.byref(eps), ctypes.byref(mu)),
+                      "fdtd_plan_materials")
+        return [None if mode.value == 0 else (("index", e[0].shape[0]) if mode.value == 1 else ("uniform", 1))
+                for mode, e in zip((eps, mu), self._compact)]
 
     def set_x_chunk(self, x_chunk):
         self.x_chunk = int(x_chunk)
@@ -353,7 +355,7 @@ class Engine:
         (0 auto, 1 inside the fused pass, 2 kernels of their own; 3 only the
         leading x/y slabs split off; 4 interior/shell partition: the fused
         pass over the box inside every slab, one kernel with every slab over
-        the shell around it), how the staged passes read the
+        the shell around it), how the passes read the
         materials (0 a one-byte index into a table of distinct value triples,
         or nothing for a uniform material, where the materials allow; 1 the
         full arrays), and whether full steps run as one pass each (0 auto:

@@ -148,8 +148,13 @@ class Grid:
         if self._H_lo is not None:
             self._H_lo.zero_()
 
+    # Changes of the material arrays in place are followed before the next call
+    # that steps the grid, by torch's count of them.  After a write that torch
+    # does not count (through .data or another library's view of the memory),
+    # assign the array to itself.
     @property
     def inverse_permittivity(self):
+        """1 / permittivity, (Nx, Ny, Nz, 3) device tensor."""
         return self._inverse_permittivity
 
     @inverse_permittivity.setter
@@ -158,6 +163,7 @@ class Grid:
 
     @property
     def inverse_permeability(self):
+        """1 / permeability, (Nx, Ny, Nz, 3) device tensor."""
         return self._inverse_permeability
 
     @inverse_permeability.setter

@@ -174,15 +174,16 @@ typedef struct {
                                          courant * inverse_permittivity / permeability (the
                                          products the reference forms first), so the kernels
                                          skip that multiply; 0 = plain inverse materials */
-    /* Optional compact copies of inv_eps / inv_mu for the TMA-staged passes
-     * (inv_eps and inv_mu stay required in full for the other kernels): a
-     * table of n value triples (plan element type) and a one-byte index per
-     * cell ([nx][ny][nz], nz a multiple of 16) with inv_eps[cell] ==
-     * table[index[cell]] for every cell; or n = 1 and index = NULL when every
-     * cell holds table[0].  The staged passes (and the PML slab kernels of
-     * such plans) then read one byte per cell, or nothing, instead of three
-     * values.  n = 0: not given.  The caller keeps the copies consistent with
-     * the full arrays; an index byte >= n reads zeros.  An index whose
+    /* Optional compact copies of inv_eps / inv_mu (which stay required in full
+     * for the kernels that do not read them): a table of n value triples (plan
+     * element type) and a one-byte index per cell ([nx][ny][nz], nz a multiple
+     * of 16) with inv_eps[cell] == table[index[cell]] for every cell; or n = 1
+     * and index = NULL when every cell holds table[0].  Staged, flat, shell and
+     * PML slab kernels and their transposes then read one byte per cell, or
+     * nothing, instead of three values; register-streaming passes use the
+     * triple of a uniform material (fdtd_plan_materials).  n = 0: not given.
+     * The caller keeps the copies consistent with the full arrays at every
+     * call, whatever the variant; an index byte >= n reads zeros.  An index whose
      * pointer is not 16-byte aligned, or nz not a multiple of 16, leaves the
      * plan on the full arrays. */
     const void *eps_table;
@@ -386,6 +387,10 @@ int fdtd_plan_step_fusion(const fdtd_plan *plan, int32_t *allowed, int32_t *acti
  * step, whose tiling is then reported; 5 the persistent loop of
  * flat or register-streaming tiles, one launch per fdtd_run call), ring stages. */
 int fdtd_plan_tiling(const fdtd_plan *plan, int64_t *out8);
+
+/* How the half steps of fdtd_run read each material: 0 the full array, 1 the
+ * one-byte index into the table, 2 the table's one triple (uniform). */
+int fdtd_plan_materials(const fdtd_plan *plan, int32_t *eps, int32_t *mu);
 
 const char *fdtd_status_string(int32_t status);
 int32_t fdtd_last_cuda_error(void);
