@@ -38,6 +38,7 @@ static bool aligned8(const void *ptr) { return ((uintptr_t)ptr & 7u) == 0; }
 
 // Cells from which a thick shell is split off automatically (see mode 4 below).
 static const long kPartition32 = 3800000, kPartition32odd = 2600000, kPartition64 = 500000, kPartition32c = 800000;
+static const long kLoop32 = 3000000;  // float32 and float32c cells below which the persistent loop runs by itself
 static const long kPartition64fit = 1L << 20, kPartition32cfit = 1300000;  // rows that fill the register tiles
 
 // Threads along z of a register-streaming tile for zt threads' worth of
@@ -708,8 +709,48 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
     GridK inside = g;  // with the layers inside the pass
     inside.nslab = ks;
     inside.nslab_fused = std::min(g.nslab_fused, ks);
-    const bool flat = !use_tma && d->precision == FDTD_FLOAT32 && p.n_shell == 0 && flat2d &&
+    // Objects that share cells: a flat thread applies them one after the other
+    // on every plane, each a chain of loads, and the blocks in them keep the
+    // others waiting, at the persistent loop's barriers most of all, whose tiles
+    // are long.  stack: objects that meet one of them; load: the planes of one
+    // tile of the loop that they take up, added up.  us per step, flat tiles in
+    // the loop, flat half steps and register tiles in the loop: 128^3 (19
+    // planes) one object 46 53 70, two 67 61 70, three 81 65 71, five 150 89 77;
+    // 104x167x145 (26 planes) one 93 71 75, two 111 76 76, three 138 82 77; 96^3
+    // (8) two 29 35 41, three 37 39 42, four 45 41 44; 64^3 (3) eight 34 34 37;
+    // 2D 900^2 (8) one 27 35 28, two 32 37 28; 400^2 (2) three 15 24 16, eight 25
+    // 30 22; 2072x291 (10) one 29 34 30, two 35 37 31.  Without the loop, flat and
+    // register half steps: 128^3 three 65 75, five 83 78, eight 113 83;
+    // 180x180x100 eight 139 141; 2D 1000^2 two 38 38, three 41 38.
+    const bool loop = d->persistent != 1 && (d->persistent == 2 || ncell < kLoop32) && p.epi_E.empty() &&
+                      p.epi_H.empty() && d->n_current_cells == 0 && d->n_dft <= kPersistMaxDft;
+    const long plane_chunks = ((long)d->ny * d->nz + kFlatBlock - 1) / kFlatBlock;
+    const int tile_planes = loop_planes(d->nx, plane_chunks, (long)PersistTune<PF32, 0>::blocks * n_sm,
+                                        flat_planes(d->nx, plane_chunks, (long)kFlatBlocks * n_sm));
+    int stack = 0;
+    long load = 0;
+    for (int a = 0; a < d->n_objects && (stack < 5 || load <= 24); ++a) {
+        int meet = 0;
+        long planes = 0;
+        for (int b = 0; b < d->n_objects; ++b) {
+            int lo[3], hi[3];
+            for (int x = 0; x < 3; ++x) {
+                lo[x] = std::max(d->objects[a].lo[x], d->objects[b].lo[x]);
+                hi[x] = std::min(d->objects[a].hi[x], d->objects[b].hi[x]);
+            }
+            if (lo[0] >= hi[0] || lo[1] >= hi[1] || lo[2] >= hi[2]) continue;
+            ++meet;
+            planes += std::min(tile_planes, hi[0] - lo[0]);
+        }
+        stack = std::max(stack, meet);
+        load = std::max(load, planes);
+    }
+    const bool heavy = load > (d->nz > 1 ? 24 : 10);
+    const bool tiles = loop ? heavy && (d->nz == 1 || stack > 2 || d->persistent == 2)
+                            : stack >= (d->nz > 1 ? 5 : 3) && ncell < kLoop32;
+    const bool flat = !use_tma && d->precision == FDTD_FLOAT32 && p.n_shell == 0 && flat2d && !tiles &&
                       flat_layers(inside, 2 * esize);
+    const bool half_steps = flat && loop && heavy;  // not in the loop
     p.flat = flat;
     if (!use_tma) {
         // (the vector tiles load auxiliaries 16 bytes at a time)
@@ -773,7 +814,7 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
             chunks = std::max(1L, std::min(chunks, std::max(1L, (long)bnx / 12)));
             t.XC = (int)((bnx + chunks - 1) / chunks);
         } else {
-            t.XC = flat ? flat_planes(bnx, flat_chunks, 4L * n_sm) : register_chunk(bnx, cols, wave);
+            t.XC = flat ? flat_planes(bnx, flat_chunks, (long)kFlatBlocks * n_sm) : register_chunk(bnx, cols, wave);
         }
     }
     t.gx = (bnx + t.XC - 1) / t.XC;
@@ -1490,7 +1531,7 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
     if (p.adj_flat) {
         const long chunks = ((long)d->ny * d->nz + kFlatBlock - 1) / kFlatBlock;
         p.kadj.flat_chunks = (unsigned)chunks;
-        p.kadj.XC = flat_planes(d->nx, chunks, 4L * n_sm);
+        p.kadj.XC = flat_planes(d->nx, chunks, (long)kFlatBlocks * n_sm);
         const long blocks = chunks * ((d->nx + p.kadj.XC - 1) / p.kadj.XC);
         p.adj_flat = blocks < (1L << 31);
         p.adj_flat_blocks = (unsigned)blocks;
@@ -1579,8 +1620,9 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
         // 55.7 -> 54.3, but 192x192x96 112 -> 135; float64 register tiles
         // 64^3 70 -> 58, 128^3 309 -> 304 (larger float64 grids with layers
         // are partitioned)
-        const long auto_cells = d->precision == FDTD_FLOAT64 ? (8L << 20) : 3000000L;
-        p.persistent = p.persist_ok && (d->persistent == 2 || (d->persistent == 0 && ncell < auto_cells));
+        const long auto_cells = d->precision == FDTD_FLOAT64 ? (8L << 20) : kLoop32;
+        p.persistent =
+            p.persist_ok && (d->persistent == 2 || (d->persistent == 0 && ncell < auto_cells && !half_steps));
         p.persist_blocks[0] = p.persist_blocks[1] = 0;
     }
     p.stats_ctas = std::max(1, std::min(4 * n_sm, FDTD_STATS_STATIC_MAX_ROWS));

@@ -384,10 +384,8 @@ static int run_persistent(Plan &p, const fdtd_run_args *a, const fdtd_capture_ar
     pa.gy = (int)p.grid.y;
     pa.gx = (int)p.grid.z;
     if (p.flat) {
-        // one tile per resident block where that keeps most of them busy, else the launch's tiles
         const long chunks = p.kf.flat_chunks;
-        const long parts = std::min((long)p.kf.nx, resident / chunks);
-        pa.planes = 2 * parts * chunks > resident ? (int)((p.kf.nx + parts - 1) / parts) : p.kf.XC;
+        pa.planes = loop_planes(p.kf.nx, chunks, resident, p.kf.XC);
         pa.gz = (int)chunks;
         pa.gy = 1;
         pa.gx = (p.kf.nx + pa.planes - 1) / pa.planes;

@@ -5,6 +5,7 @@
 
 #include <cuda.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "fdtd_common.cuh"
@@ -24,6 +25,14 @@ struct EpiOp {
 
 // Tensor maps of the TMA-staged kernels (one 2D view per field and box shape).
 enum MapId { MAP_H_NBR = 0, MAP_E_NBR, MAP_E_OWN, MAP_H_OWN, MAP_IE, MAP_MU, MAP_ELO, MAP_HLO, MAP_COUNT };
+
+// Planes per flat tile of the persistent loop: one tile per resident block where
+// that keeps most of them busy, else the launch's.
+inline int loop_planes(int nx, long chunks, long resident, int planes) {
+    const long parts = std::min((long)nx, resident / chunks);
+    return 2 * parts * chunks > resident ? (int)((nx + parts - 1) / parts) : planes;
+}
+
 
 struct Plan {
     int precision;
