@@ -374,8 +374,11 @@ __global__ void __launch_bounds__(kFlatBlock, 4) k_adj_flat(const __grid_constan
                 layer(1);
                 layer(2);
             } else {
+                int o = g.lay_order;
+                if (o == kOrderBySide)
+                    o = cell_order(g.lay_rank, i >= g.lay[0][0].th, j >= g.lay[1][0].th, k >= g.lay[2][0].th);
 #pragma unroll 1
-                for (int o = flat_order(g, i, j, k), r = 0; r < 3; ++r, o >>= 4) layer(o & 15);
+                for (int r = 0; r < 3; ++r, o >>= 4) layer(o & 15);
             }
             pf[0] = v.f0;
             pf[1] = v.f1;
