@@ -75,10 +75,11 @@ static bool flat_layers(GridK &g, size_t pair) {
 // two planes more for its set-up.  Up to four waves count whole (a part-filled
 // last wave takes as long as a full one); at most 12 planes, or 16 in a single
 // wave, since blocks in layers are slower and long marches leave the last of
-// them alone.  us per step, float32: 128^3 16 planes (0.84 waves) 43, 8 (1.7)
-// 46, 12 (1.2) 49; 192x192x96 12 (1.9) 110, 16 (1.4) 121, 24 (0.95) 111;
-// 256^3 4, 8, 12, 16 planes 310, 301, 301, 304; 384x384x192 16 planes 665,
-// 23 765; 2D 4000^2 8, 12, 16, 32, 64 planes 273, 275, 281, 297, 315.
+// them alone.  us per step, float32 with 10-cell layers: 128^3 16 planes (0.84
+// waves) 38, 8 (1.7) 39, 12 (1.2) 42; 192x192x96 12 (1.9) 65, 16 (1.4) 73, 24
+// (0.95) 64; 256^3 4, 8, 12, 16, 24 planes 310, 293, 287, 289, 297; 384x384x192
+// 8 to 16 planes 468, 23 472; 2D 4000^2 4, 8, 12, 16, 32, 64 planes 238, 231,
+// 226, 231, 248, 262.
 static int flat_planes(int nx, long chunks, long wave) {
     double best = 0.0;
     int planes = 1;
@@ -746,7 +747,7 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
         load = std::max(load, planes);
     }
     const bool heavy = load > (d->nz > 1 ? 24 : 10);
-    const bool tiles = loop ? heavy && (d->nz == 1 || stack > 2 || d->persistent == 2)
+    const bool tiles = loop ? heavy && (d->nz == 1 || stack > 2)
                             : stack >= (d->nz > 1 ? 5 : 3) && ncell < kLoop32;
     const bool flat = !use_tma && d->precision == FDTD_FLOAT32 && p.n_shell == 0 && flat2d && !tiles &&
                       flat_layers(inside, 2 * esize);
@@ -1616,10 +1617,11 @@ static int create(const fdtd_grid_desc *d, Plan &p) {
                        p.n_current == 0 && (int)p.dft.size() <= kPersistMaxDft;
         // automatic: float32 and float32c below 3M cells, float64 below 8M.
         // Against one launch per half step, flat tiles, us per step: 64^3
-        // 25.9 -> 12.5, 2D 1500x1100 43 -> 32, 128^3 55.6 -> 48.3, 131x150x97
-        // 55.7 -> 54.3, but 192x192x96 112 -> 135; float64 register tiles
-        // 64^3 70 -> 58, 128^3 309 -> 304 (larger float64 grids with layers
-        // are partitioned)
+        // 24.9 -> 11.9, 2D 1500x1100 42 -> 29, 128^3 53 -> 47, 131x150x97 55 ->
+        // 48, 136x132x128 (2.3M) 53 -> 43, 140^3 (2.7M) 70 -> 61, 143x150x139
+        // (3.0M) 77 -> 67, 2D 1700^2 60 -> 51, 60x200x200 60 -> 60, but
+        // 192x192x96 (3.5M) 92 -> 108; float64 register tiles 64^3 70 -> 58, 128^3
+        // 309 -> 304 (larger float64 grids with layers are partitioned)
         const long auto_cells = d->precision == FDTD_FLOAT64 ? (8L << 20) : kLoop32;
         p.persistent =
             p.persist_ok && (d->persistent == 2 || (d->persistent == 0 && ncell < auto_cells && !half_steps));
