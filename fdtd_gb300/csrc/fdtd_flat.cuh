@@ -11,16 +11,17 @@
 // / thread_H, and so are the bits.
 //
 // Bound by latency and instruction issue, not by bytes: at 128^3 with 12-cell
-// layers (everything in L2) a half step issues 207 (E) and 167 (H) warp
-// instructions per 32 cells, 47 and 36 % of the issue slots.  Four blocks of 64 registers per SM: five
-// (48 registers) and three (80, two planes in flight in every loop) measured
-// slower, 56 and 59 against 43 us per step.  Against the register-streaming
-// tiles (four cells per thread, whose warps all hold a few cells of each z
-// layer and whose 124 registers leave 16 warps per SM), float32, us per step:
-// 128^3 87 -> 53, 131x150x97 72 -> 56, 64^3 16.0 -> 14.4, 192x192x96 176 ->
-// 115.  With double or compensated values, and on the slab-free interior of a
-// partition, those stay faster: 256^3 float64 1416 against 1675, float32c 500
-// against 565.
+// layers (everything in L2) a half step issues 205 (E) and 160 (H) warp
+// instructions per 32 cells, 48 % of the issue slots.  us per step with one
+// launch per half step (plain object, plane source, plane record), four blocks
+// of 64 registers per SM: 52.8; five (48 registers) and three (80) measured 65
+// and 77.  Against the register-streaming tiles (four cells per thread, whose
+// warps all hold a few cells of each z layer and whose 124 registers leave 16
+// warps per SM), the same scene 91 -> 53, 192x192x96 169 -> 92, 131x150x97 83 ->
+// 55; in the persistent loop 128^3 89 -> 47, 64^3 15.9 -> 11.9, 131x150x97 71 ->
+// 48.  Float32 only: with double or compensated values, and on the slab-free
+// interior of a partition, the register tiles stay faster (256^3 float64 1416
+// against 1675, float32c 500 against 565).
 #pragma once
 
 #include "fdtd_cell.cuh"
