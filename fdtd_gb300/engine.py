@@ -47,7 +47,8 @@ _MAX_TABLE = 256  # distinct value triples a one-byte material index can address
 
 
 def compact_material(x, chunk=1 << 25, index_ok=True):
-    """Compact copy of a (nx, ny, nz, 3) inverse-material array: ``(table, index)`` with ``table`` an (n, 3) array of value triples
+    """Compact copy of a (nx, ny, nz, 3) inverse-material array:
+    ``(table, index)`` with ``table`` an (n, 3) array of value triples
     and ``index`` the uint8 (nx, ny, nz) table row of every cell, or
     ``(table, None)`` when every cell holds the same triple; ``None`` when the
     cells hold more than 256 distinct triples, or more than one and
